@@ -1987,6 +1987,7 @@ void lv_engine_destroy(lv_engine* E) {
   if (E->ev1) cudaEventDestroy(E->ev1);
   if (E->st) counted_sync(E->st);  // the frees above are stream-ordered
   if (E->pool) cudaMemPoolDestroy(E->pool);
+  release_sort_scratch(E->device);
   if (E->own_stream && E->st) cudaStreamDestroy(E->st);
   delete E;
 }

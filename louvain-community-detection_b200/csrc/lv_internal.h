@@ -496,13 +496,16 @@ cudaError_t configure_contract_kernels();
 // sort.cu
 // ---------------------------------------------------------------------------
 // Stable LSD radix sort of (key, u32 value) pairs on the low key_bits bits;
-// the result is in keys/vals, or in keys_alt/vals_alt when *result_in_alt.
+// the result is in keys/vals, or in keys_alt/vals_alt when *result_in_alt
+// (u64 keys).
 // counts needs radix_sort_scratch_words(n) words, S a scan of that size.
 size_t radix_sort_scratch_words(uint64_t n);
 template <typename K>
 cudaError_t radix_sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt,
                              uint64_t n, int key_bits, uint32_t* counts, ScanScratch& S,
                              cudaStream_t st, bool* result_in_alt);
+// Gives back the sorts' unused scratch on a device (kept between calls).
+void release_sort_scratch(int device);
 // CSR of an edge list with the reference reader's layout (utils.cu:168-229):
 // every row in file order, an off-diagonal edge stored in both rows, a
 // self-loop once, |w| (1 without weights).  col/wout need room for 2m
