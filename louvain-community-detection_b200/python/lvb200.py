@@ -434,10 +434,10 @@ class Engine:
         """(offsets, members) of the final partition, grouped on the device."""
         c = _U32()
         _check(lib().lv_get_communities(self._h, None, 0, ctypes.byref(c)))
-        out = np.zeros(int(c.value) + 1 + self.n0, dtype=np.uint32)
+        out = np.empty(int(c.value) + 1 + self.n0, dtype=np.uint32)
         _check(lib().lv_get_communities(self._h, _p(out), out.size, ctypes.byref(c)))
         k = int(c.value)
-        return out[:k + 1].copy(), out[k + 1:].copy()
+        return out[:k + 1], out[k + 1:]  # the two parts of one array of their own
 
     def load_device(self, n: int, nnz: int, d_off: int, d_col: int, d_w: int):
         _check(lib().lv_engine_load_device(self._h, n, nnz, d_off, d_col, d_w))
