@@ -2537,16 +2537,17 @@ lv_status lv_modularity_fp64(lv_engine* E, const uint32_t* partition, double* q)
   if (!E || !partition || !q) return fail(LV_ERR_ARG, "NULL argument");
   if (!E->loaded) return fail(LV_ERR_STATE, "no graph loaded");
   cudaSetDevice(E->device);
-  for (uint32_t i = 0; i < E->n; i++)
-    if (partition[i] >= E->n) return fail(LV_ERR_ARG, "community id out of range");
+  // contraction scratch, idle between entry points
   uint32_t* d_part = E->cb.cursor;
   double* d_tot = reinterpret_cast<double*>(E->cb.comm_deg);
-  double* d_out = reinterpret_cast<double*>(E->cb.new_deg);
+  double* d_out = reinterpret_cast<double*>(E->cb.counts);  // 4 of its 16 words' 8 doubles
   if (E->n) CU(cudaMemcpyAsync(d_part, partition, (size_t)E->n * 4, cudaMemcpyHostToDevice, E->st));
-  CU(launch_modularity_of(E->view(), d_part, d_tot, d_out, E->st));
-  double h[3] = {0, 0, 0};
+  CU(launch_modularity_of(E->view(), d_part, d_tot, d_out, E->cb.members, E->cb.comm_list,
+                          E->cb.counts + 15, E->st));
+  double h[4] = {0, 0, 0, 0};
   CU(cudaMemcpyAsync(h, d_out, sizeof(h), cudaMemcpyDeviceToHost, E->st));
   CU(counted_sync(E->st));
+  if (h[3] != 0.0) return fail(LV_ERR_ARG, "community id out of range");
   const double m = h[2] / 2.0;
   *q = (m > 0.0) ? h[0] / (2.0 * m) - h[1] / (4.0 * m * m) : 0.0;
   return LV_OK;

@@ -478,10 +478,13 @@ cudaError_t launch_add_u32(uint32_t* a, size_t n, uint32_t d, cudaStream_t st);
 cudaError_t launch_add_u64(uint64_t* a, size_t n, uint64_t d, cudaStream_t st);
 // Recompute sizes and totals from comm (used when a caller sets comm).
 cudaError_t launch_recount(const LevelView& L, cudaStream_t st);
-// FP64 modularity of an arbitrary partition (one-off, not hot).
+// FP64 modularity of an arbitrary partition: out[0..3] the intra-community
+// weight, the squared totals, the total weight and how many vertices have a
+// community id >= n (those are left out).  Scratch: tot_scratch, list_row and
+// list_chunk of n elements, list_cnt of one.
 cudaError_t launch_modularity_of(const LevelView& L, const uint32_t* part,
-                                 double* tot_scratch, double* out,
-                                 cudaStream_t st);
+                                 double* tot_scratch, double* out, uint32_t* list_row,
+                                 uint32_t* list_chunk, uint32_t* list_cnt, cudaStream_t st);
 cudaError_t launch_bucket_ids(const uint64_t* off, uint32_t n, uint8_t* out,
                               cudaStream_t st);
 unsigned dispatch_grid(const DispatchPlan& P);
