@@ -370,6 +370,13 @@ struct lv_engine {
   // returned true or a caller set them; `assignment` itself holds the
   // level-start map and is composed once per level, at aggregation.
   bool accepted = false;
+  // the level's state came from the small-run kernel: no class lists, plan or
+  // row ids were built for it (refresh_plan builds them)
+  bool plan_stale = false;
+  // small-run kernel: its buffers (one allocation) and pinned result
+  unsigned char* small_buf = nullptr;
+  SmallRunResult* small_host = nullptr;
+  bool small_off = false;  // the device cannot run it
   DispatchPlan plan{};
   double q_last = 0.0;
   std::vector<lv_level_info> levels;
@@ -950,9 +957,8 @@ lv_status prepare_level(lv_engine* E, bool sync_scalars = true) {
     prof_collect(E);
   }
   g_trace.mark("  level init + Q0", (uint32_t)E->levels.size(), n);
-  // tables of E->n vertices (blocking host copies above must be done
-  // before the vectors go out of scope: synchronised)
   E->level_ready = true;
+  E->plan_stale = false;
   return LV_OK;
 }
 
@@ -1295,6 +1301,7 @@ lv_status load_common(lv_engine* E, uint32_t n, uint64_t e) {
   E->cur = -1;
   E->loaded = true;
   E->level_ready = false;
+  E->plan_stale = false;
   E->finished = false;
   E->accepted = false;
   E->batch = false;
@@ -1941,6 +1948,7 @@ lv_status lv_engine_create(const lv_config* cfg, lv_engine** out) {
       (ce = cudaEventCreateWithFlags(&E->desc_ev, cudaEventDisableTiming)) != cudaSuccess ||
       (ce = cudaMallocHost(&E->desc_host, sizeof(PassDesc))) != cudaSuccess ||
       (ce = cudaEventCreate(&E->agg_ev1)) != cudaSuccess ||
+      (ce = cudaMallocHost(&E->small_host, sizeof(SmallRunResult))) != cudaSuccess ||
       (ce = cudaMallocHost(&E->h_pending, 2 * sizeof(uint64_t))) != cudaSuccess) {
     lv_engine_destroy(E);
     return cuda_fail(ce, "engine set-up");
@@ -1972,6 +1980,8 @@ void lv_engine_destroy(lv_engine* E) {
   for (cudaEvent_t ev : E->ev_free) cudaEventDestroy(ev);
   E->ev_free.clear();
   dfree(E->d_class_deg);
+  dfree(E->small_buf);
+  if (E->small_host) cudaFreeHost(E->small_host);
   if (E->sc) cudaFree(E->sc);
   if (E->d_desc) cudaFree(E->d_desc);
   if (E->loop_state) cudaFree(E->loop_state);
@@ -2100,6 +2110,134 @@ lv_status lv_engine_load_device(lv_engine* E, uint32_t n, uint64_t nnz,
   return load_common(E, n, nnz);
 }
 
+// ---------------------------------------------------------------------------
+// Small levels of a single graph (small_run.cuh)
+// ---------------------------------------------------------------------------
+// Entries a level may have for the small-run kernel.  Its 16 SMs take longer
+// over a pass than the level graph's launches do from about 12 K entries on
+// (LFR, 9.7 K entries: 39 against 43 us a pass; 21 K: 49 against 44; R-MAT,
+// 45 K: 155 against 64), but a level's set-up, contraction and host waits
+// cost 40 us instead of 250: a contracted level, which has a few passes,
+// gains up to about 32 K.  One block, without cluster barriers, for the
+// smallest (where the entries are not known yet: by vertices).
+constexpr uint64_t kSmallFirstEntries = 12288;
+constexpr uint64_t kSmallLaterEntries = 32768;
+constexpr uint64_t kSmallOneEntries = 1536;
+constexpr uint32_t kSmallOneVertices = 64;
+
+static uint64_t small_max_entries(const lv_engine* E) {
+  return E->levels.empty() ? kSmallFirstEntries : kSmallLaterEntries;
+}
+
+// A level the small-run kernel may take: the default single-graph path, not
+// set up yet.  Its entry count may still be on the device (agg_pending): the
+// kernel then refuses a level with too many.
+static bool small_eligible(const lv_engine* E) {
+  return E->cfg.use_graphs && !E->profiling && !E->batch && !use_level_kernel(E) &&
+         !E->cfg.contract_sort && !E->cfg.apply_launch && !E->level_ready && !E->small_off &&
+         E->n > 0 && E->n <= kSmallMaxN && (E->agg_pending || E->e <= small_max_entries(E));
+}
+
+// Runs the engine's level (with move_only its passes, else every level to the
+// end of the run) in the small-run kernel and waits for it; *took = false
+// when the kernel did not take the level, whose entry count is known then.
+static lv_status small_run(lv_engine* E, float min_gain, bool move_only, bool* took) {
+  *took = false;
+  cudaStream_t st = E->st;
+  constexpr size_t kIds = (size_t)kSmallMaxN * sizeof(uint32_t);
+  if (!E->small_buf) CU(dalloc(&E->small_buf, kIds + 256 + sizeof(SmallRunResult)));
+  unsigned char* b = E->small_buf;
+  SmallRunArgs a{};
+  a.L = E->view();
+  a.e_dev = E->agg_pending ? reinterpret_cast<const uint64_t*>(E->cb.counts + 8) : nullptr;
+  a.e = E->e;
+  a.e_max = small_max_entries(E);
+  a.cur = E->cur;
+  for (int i = 0; i < 2; i++) {
+    a.c_off[i] = E->c_off[i];
+    a.c_col[i] = E->c_col[i];
+    a.c_w[i] = E->c_w[i];
+  }
+  const ContractBuffers& B = E->cb;
+  a.tcol = B.tcol;
+  a.tw = B.tw;
+  a.seg = B.seg;
+  a.new_deg = B.new_deg;
+  a.map = reinterpret_cast<uint32_t*>(b);
+  a.counters = reinterpret_cast<uint32_t*>(b + kIds);
+  a.res = reinterpret_cast<SmallRunResult*>(b + kIds + 256);
+  a.min_gain = (double)min_gain;
+  a.max_passes = E->cfg.max_passes;
+  a.max_levels = E->cfg.max_levels ? E->cfg.max_levels - (uint32_t)E->levels.size() : 0u;
+  a.move_only = move_only ? 1u : 0u;
+  const bool one = E->n <= kSmallOneMaxN &&
+                   (E->agg_pending ? E->n <= kSmallOneVertices : E->e <= kSmallOneEntries);
+  const cudaError_t ce = launch_small_run(a, engine_mode(E), one, st);
+  if (ce == cudaErrorNotSupported) {
+    E->small_off = true;
+    return LV_OK;
+  }
+  CU(ce);
+  SmallRunResult* R = E->small_host;
+  CU(cudaMemcpyAsync(R, a.res, sizeof(SmallRunResult), cudaMemcpyDeviceToHost, st));
+  CU(cudaMemcpyAsync(E->sc_host, E->sc, sizeof(LevelScalars), cudaMemcpyDeviceToHost, st));
+  if (E->agg_pending)
+    CU(cudaMemcpyAsync(E->h_pending, E->cb.counts + 8, sizeof(uint64_t), cudaMemcpyDeviceToHost,
+                       st));
+  CU(counted_sync(st));
+  LVTRY(finish_pending(E));
+  LVTRY(check_device_error(E));
+  g_trace.mark("small run", R->levels, E->n);
+  if (R->status == kSmallRefused || (R->status == kSmallMore && R->levels == 0)) return LV_OK;
+  *took = true;
+  for (uint32_t i = 0; i < R->levels; i++) {
+    const SmallLevel& l = R->level[i];
+    lv_level_info info{};
+    info.n_vertices = l.n;
+    info.n_entries = l.e;
+    info.passes = l.passes;
+    info.moved = (R->status == kSmallFirstFail && i + 1 == R->levels) ? 0u : 1u;
+    info.q_start = l.q_start;
+    info.q_end = l.q_end;
+    info.move_ms = (float)((double)(l.t_moved - l.t_start) * 1e-6);
+    info.prepare_ms = (float)((double)(l.t_ready - l.t_start) * 1e-6);
+    info.aggregate_ms = (float)((double)(l.t_done - l.t_moved) * 1e-6);
+    E->levels.push_back(info);
+  }
+  if (R->contracted) CU(launch_compose(E->assignment, E->n0, a.map, st));
+  E->cur = R->cur;
+  E->n = R->n;
+  E->e = R->e;
+  E->q_last = R->q;
+  E->accepted = false;
+  // the level it ended in keeps its state, as after a level graph; a level it
+  // stopped before is not set up
+  E->level_ready = move_only || R->status == kSmallFirstFail;
+  E->plan_stale = E->level_ready;
+  if (R->status == kSmallFirstFail || R->status == kSmallMerged0) E->finished = true;
+  return LV_OK;
+}
+
+// Class lists and plan of a level whose state came from the small-run
+// kernel; the state itself stays as it is.
+static lv_status refresh_plan(lv_engine* E) {
+  if (!E->plan_stale) return LV_OK;
+  const size_t n = E->n;
+  CU(cudaMemcpyAsync(E->cb.cursor, E->comm, n * 4, cudaMemcpyDeviceToDevice, E->st));
+  LVTRY(prepare_level(E));
+  CU(cudaMemcpyAsync(E->comm, E->cb.cursor, n * 4, cudaMemcpyDeviceToDevice, E->st));
+  CU(launch_recount(E->view(), E->st));
+  CU(cudaMemcpyAsync(E->comm_alt, E->comm, n * 4, cudaMemcpyDeviceToDevice, E->st));
+  CU(cudaMemcpyAsync(E->sz_alt, E->comm_sz, n * 4, cudaMemcpyDeviceToDevice, E->st));
+  CU(cudaMemcpyAsync(E->tot_alt, E->tot, n * 8, cudaMemcpyDeviceToDevice, E->st));
+  CU(cudaMemcpyAsync(E->comm_start, E->comm, n * 4, cudaMemcpyDeviceToDevice, E->st));
+  CU(launch_modularity(E->view(), E->order, E->plan,
+                       E->plan.hub_count ? E->hub_map : nullptr, E->partials, E->st));
+  CU(cudaMemcpyAsync(E->sc_host, E->sc, sizeof(LevelScalars), cudaMemcpyDeviceToHost, E->st));
+  CU(counted_sync(E->st));
+  return LV_OK;
+}
+
 // A level's move phase.  With `speculate` (the whole-run loop of a single
 // graph), the contraction's front is launched behind the level graph
 // before its result is known, and one synchronisation reads both: the
@@ -2113,6 +2251,18 @@ static lv_status phase_move(lv_engine* E, float min_gain, int* more, double* q,
   if (E->finished) return fail(LV_ERR_STATE, "the run has ended; load a graph again");
   cudaSetDevice(E->device);
   E->front_ready = false;
+  if (!speculate && small_eligible(E)) {  // the whole-run loop asks by itself
+    bool took = false;
+    LVTRY(small_run(E, min_gain, true, &took));
+    if (took) {
+      const bool moved = E->levels.back().moved != 0;
+      E->accepted = moved;
+      if (more) *more = moved ? 1 : 0;
+      if (q) *q = E->q_last;
+      return LV_OK;
+    }
+  }
+  if (E->level_ready) LVTRY(refresh_plan(E));  // more passes on the same level
   CU(cudaEventRecord(E->ev0, E->st));
   g_trace.reset();
   // the level graph reads the level's m and initial Q on the device and the
@@ -2305,6 +2455,22 @@ static lv_status run_loaded(lv_engine* E, float min_gain, lv_result* res) {
   uint64_t processed = 0;
   for (;;) {
     int more = 0;
+    if (small_eligible(E)) {
+      bool took = false;
+      const size_t first = E->levels.size();
+      const lv_status s = small_run(E, min_gain, false, &took);
+      if (s != LV_OK) {
+        cudaEventDestroy(a0);
+        cudaEventDestroy(a1);
+        return s;
+      }
+      for (size_t i = first; i < E->levels.size(); i++)
+        processed += (uint64_t)E->levels[i].passes * E->levels[i].n_entries;
+      if (took) {
+        q = E->q_last;
+        if (E->finished) break;
+      }
+    }
     lv_status s = phase_move(E, min_gain, &more, &q, true);
     if (s != LV_OK) {
       cudaEventDestroy(a0);
@@ -2512,7 +2678,7 @@ lv_status lv_set_level_comm(lv_engine* E, const uint32_t* comm) {
   cudaSetDevice(E->device);
   for (uint32_t i = 0; i < E->n; i++)
     if (comm[i] >= E->n) return fail(LV_ERR_ARG, "community id out of range");
-  if (!E->level_ready) LVTRY(prepare_level(E));
+  if (!E->level_ready || E->plan_stale) LVTRY(prepare_level(E));
   if (E->n) CU(cudaMemcpyAsync(E->comm, comm, (size_t)E->n * 4, cudaMemcpyHostToDevice, E->st));
   CU(launch_recount(E->view(), E->st));
   if (E->n) {  // the second copy of the state starts equal to the first
@@ -2960,6 +3126,7 @@ lv_status lv_autotune(lv_engine* E, uint32_t reps, lv_tuning* out) {
   cudaSetDevice(E->device);
   if (!reps) reps = 5;
   if (!E->level_ready) LVTRY(prepare_level(E));
+  LVTRY(refresh_plan(E));
   drop_pass_graph(E);  // a captured pass would keep the old kernels
   LVTRY(upload_desc(E, 0.0f));
   const int rule = engine_mode(E);

@@ -496,6 +496,56 @@ cudaError_t configure_kernels();
 cudaError_t configure_contract_kernels();
 
 // ---------------------------------------------------------------------------
+// small_run.cuh: the remaining levels of a small single graph in one launch
+// ---------------------------------------------------------------------------
+constexpr uint32_t kSmallMaxN = 2048;    // vertices of a level it takes
+constexpr uint32_t kSmallOneMaxN = 1024;  // as one block
+constexpr uint32_t kSmallLevels = 32;   // levels of one launch
+enum SmallRunStatus : uint32_t {
+  kSmallRefused = 0,   // the first level does not fit: nothing was done
+  kSmallMore = 1,      // stopped at a level boundary: that level runs elsewhere
+  kSmallFirstFail = 2, // a level's first pass gained too little: the run ends
+  kSmallMerged0 = 3,   // a level merged nothing, or the level limit: it ends
+};
+struct SmallLevel {
+  uint32_t n, passes;
+  uint64_t e;
+  double q_start, q_end;
+  unsigned long long t_start, t_ready, t_moved, t_done;  // nanoseconds
+};
+struct SmallRunResult {
+  uint32_t status, levels;  // SmallRunStatus; levels finished by this launch
+  uint32_t n;               // the level it stopped at
+  uint64_t e;
+  int32_t cur;              // CSR buffer of that level (-1: the input)
+  uint32_t contracted;      // levels contracted (map is to be composed if > 0)
+  double q;                 // the run's modularity so far (modularity.cu:503-517)
+  SmallLevel level[kSmallLevels];
+};
+struct SmallRunArgs {
+  LevelView L;              // the level (n, CSR) and the engine's state arrays
+  const uint64_t* e_dev;    // the level's entry count where the host does not
+  uint64_t e, e_max;        // know it yet (else nullptr and e); largest taken
+  int32_t cur;              // -1, 0, 1
+  uint64_t* c_off[2];       // the engine's contracted CSR buffers
+  uint32_t* c_col[2];
+  float* c_w[2];
+  uint32_t* tcol;           // row staging, as in ContractBuffers
+  float* tw;
+  uint64_t *seg, *new_deg;
+  uint32_t* map;            // [kSmallMaxN] first level's vertex -> current vertex
+  uint32_t* counters;       // [2] staging bumps, zeroed by the kernel
+  SmallRunResult* res;
+  double min_gain;
+  uint32_t max_passes, max_levels;  // levels this run may still do (0: no cap)
+  uint32_t move_only;       // stop after the first level's passes
+};
+// One block (levels of at most kSmallOneMaxN vertices), or one cluster of 16
+// (8 where the device cannot co-schedule 16).  cudaErrorNotSupported: the
+// device cannot run it.
+cudaError_t launch_small_run(const SmallRunArgs& A, int mode, bool one, cudaStream_t st);
+
+// ---------------------------------------------------------------------------
 // sort.cu
 // ---------------------------------------------------------------------------
 // Stable LSD radix sort of (key, u32 value) pairs on the low key_bits bits;

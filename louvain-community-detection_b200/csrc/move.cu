@@ -495,7 +495,7 @@ __device__ __forceinline__ void record_decision(const PassDesc* __restrict__ D,
 // memory from the caller: the standalone kernels pass blockIdx/gridDim and
 // their own shared arrays, the persistent level kernel the same body with
 // its one shared-memory arena.
-template <int G, int MODE>
+template <int G, int MODE, int NT = kThreads>
 __device__ __forceinline__ void small_body(const PassDesc* __restrict__ D, int cls,
                                            uint32_t bid, uint32_t nblk, double (*sums)[32],
                                            const StepIO io = StepIO{}) {
@@ -511,9 +511,10 @@ __device__ __forceinline__ void small_body(const PassDesc* __restrict__ D, int c
   const uint32_t count = D->act_cnt ? D->act_cnt[cls] : D->A.P.cls_start[cls + 1] - s0;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int gl = lane & (G - 1);
-  const uint32_t per_block = kThreads / G;
+  const uint32_t per_block = NT / G;
   for (uint32_t base = bid * per_block; base < count; base += nblk * per_block) {
     const uint32_t vidx = base + threadIdx.x / G;
+    if (base + (threadIdx.x & ~31u) / G >= count) break;  // a warp without vertices
     const bool vvalid = vidx < count;
     uint32_t v = 0, d = 0, cv = 0;
     uint64_t s = 0;
@@ -636,7 +637,9 @@ template <int NV, int NT>
 __device__ __forceinline__ uint64_t vec_entry(uint64_t s, uint32_t t, int i) {
   return ((s >> 2) + (uint64_t)(i >> 2) * NT + t) * 4 + (uint64_t)(i & 3);
 }
-template <int NV, int NT>
+// COHERENT: plain loads instead of the read-only path, for a kernel that
+// rewrites the CSR buffers between its levels.
+template <int NV, int NT, bool COHERENT = false>
 __device__ __forceinline__ void load_row_vec(const LevelView& L, uint64_t s, uint64_t e_end,
                                              uint32_t t, uint32_t fill, bool vec_ok,
                                              uint32_t (&cu)[4 * NV], float (&wt)[4 * NV]) {
@@ -644,8 +647,10 @@ __device__ __forceinline__ void load_row_vec(const LevelView& L, uint64_t s, uin
   for (int k = 0; k < NV; k++) {
     const uint64_t base = vec_entry<NV, NT>(s, t, 4 * k);
     if (vec_ok && base >= s && base + 4 <= e_end) {
-      const uint4 c = __ldg(reinterpret_cast<const uint4*>(L.col) + (base >> 2));
-      const float4 w = __ldg(reinterpret_cast<const float4*>(L.w) + (base >> 2));
+      const uint4* cp = reinterpret_cast<const uint4*>(L.col) + (base >> 2);
+      const float4* wp = reinterpret_cast<const float4*>(L.w) + (base >> 2);
+      const uint4 c = COHERENT ? *cp : __ldg(cp);
+      const float4 w = COHERENT ? *wp : __ldg(wp);
       cu[4 * k] = c.x;
       cu[4 * k + 1] = c.y;
       cu[4 * k + 2] = c.z;
@@ -727,11 +732,13 @@ __device__ __forceinline__ typename BestOf<PREC>::T eval_own_slot(
 
 // 32 < deg <= 319: one warp per vertex, T-slot table per warp.  All of a
 // row's loads (at most MAXW waves of 32) are issued before any insertion,
-// so a vertex costs one memory latency chain instead of one per wave.
-template <int T, int MAXW, int MODE>
+// so a vertex costs one memory latency chain instead of one per wave.  nw:
+// the block's warps that have a table (its first ones).
+template <int T, int MAXW, int MODE, bool COHERENT = false>
 __device__ __forceinline__ void warp_body(const PassDesc* __restrict__ D, int cls, uint32_t bid,
                                           uint32_t nblk, unsigned char* smem_raw,
-                                          const StepIO io = StepIO{}) {
+                                          const StepIO io = StepIO{},
+                                          const uint32_t nw = kWarps) {
   constexpr int RULE = ModeOf<MODE>::kRule, PREC = ModeOf<MODE>::kPrec;
   const LevelView L = step_view(D, io);
   reapply_prev_step(D, io, bid, nblk);
@@ -742,11 +749,11 @@ __device__ __forceinline__ void warp_body(const PassDesc* __restrict__ D, int cl
   const uint32_t count = D->act_cnt ? D->act_cnt[cls] : D->A.P.cls_start[cls + 1] - s0;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   double* vals = reinterpret_cast<double*>(smem_raw) + wib * T;
-  uint32_t* keys =
-      reinterpret_cast<uint32_t*>(smem_raw + sizeof(double) * T * kWarps) + wib * T;
+  uint32_t* keys = reinterpret_cast<uint32_t*>(smem_raw + sizeof(double) * T * nw) + wib * T;
   uint32_t clean = 0;  // leading table slots known to be empty
+  if (COHERENT && (uint32_t)wib >= nw) return;
   const bool vec_ok = (((uintptr_t)L.col | (uintptr_t)L.w) & 15u) == 0;
-  for (uint32_t vidx = bid * kWarps + wib; vidx < count; vidx += nblk * kWarps) {
+  for (uint32_t vidx = bid * nw + wib; vidx < count; vidx += nblk * nw) {
     const uint32_t v = verts[vidx];
     const uint64_t s = L.off[v];
     const uint32_t d = (uint32_t)(L.off[v + 1] - s);
@@ -782,7 +789,7 @@ __device__ __forceinline__ void warp_body(const PassDesc* __restrict__ D, int cl
       return kVec ? vec_entry<NV, 32>(s, ln, i) : s + (uint64_t)i * 32 + ln;
     };
     if constexpr (kVec) {
-      load_row_vec<NV, 32>(L, s, e_end, lane, v, vec_ok, cu, wt);
+      load_row_vec<NV, 32, COHERENT>(L, s, e_end, lane, v, vec_ok, cu, wt);
     } else {
 #pragma unroll
       for (int i = 0; i < NE; i++) {
@@ -872,7 +879,7 @@ __device__ __forceinline__ double block_sum(double x, double* red) {
 // registers -- every load issued before any is used -- then inserts them
 // into a table (clear it before, synchronise after).  cu / wt / owned come
 // back as eval_owned reads them.
-template <int MAXW, int RULE>
+template <int MAXW, int RULE, int NT>
 __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t s,
                                                    uint64_t lo, uint64_t end,
                                                    uint32_t v, uint32_t cv,
@@ -887,7 +894,7 @@ __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t 
   owned = 0u;
 #pragma unroll
   for (int k = 0; k < MAXW; k++) {
-    const uint64_t j = lo + (uint64_t)k * kThreads + threadIdx.x;
+    const uint64_t j = lo + (uint64_t)k * NT + threadIdx.x;
     cu[k] = v;
     wt[k] = 0.0f;
     if (j < end) {
@@ -897,14 +904,14 @@ __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t 
   }
 #pragma unroll
   for (int k = 0; k < MAXW; k++) {
-    const uint64_t j = lo + (uint64_t)k * kThreads + threadIdx.x;
+    const uint64_t j = lo + (uint64_t)k * NT + threadIdx.x;
     if (cu[k] == v) self_mask |= 1u << k;
     cu[k] = (j < end) ? L.comm[cu[k]] : kEmptyKey;
   }
 #pragma unroll
   for (int k = 0; k < MAXW; k++) {
-    if (lo + (uint64_t)k * kThreads >= end) break;  // block-uniform
-    const bool has = lo + (uint64_t)k * kThreads + threadIdx.x < end;
+    if (lo + (uint64_t)k * NT >= end) break;  // block-uniform
+    const bool has = lo + (uint64_t)k * NT + threadIdx.x < end;
     // own-community entries go to the caller's register sum (hot)
     const bool is_hot = has && cu[k] == cv;
     const bool ins = has && !is_hot;
@@ -922,7 +929,7 @@ __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t 
   }
 }
 
-template <int MODE>
+template <int MODE, int NT = kThreads>
 __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int cls, uint32_t bid,
                                            uint32_t nblk, unsigned char* smem_raw,
                                            typename BestOf<ModeOf<MODE>::kPrec>::T* red_best,
@@ -937,7 +944,7 @@ __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int c
   uint32_t* __restrict__ prop = D->prop + s0;
   const uint32_t count = D->act_cnt ? D->act_cnt[cls] : D->A.P.cls_start[cls + 1] - s0;
   constexpr int T = kHubSmemSlots;
-  constexpr int MAXW = (int)(kHubSmemMaxDeg / kThreads);
+  constexpr int MAXW = (int)(kHubSmemMaxDeg / NT);
   double* vals = reinterpret_cast<double*>(smem_raw);
   uint32_t* keys = reinterpret_cast<uint32_t*>(smem_raw + sizeof(double) * T);
   uint32_t clean = 0;  // leading table slots known to be empty
@@ -954,7 +961,7 @@ __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int c
     }
     const uint32_t tv = table_size_for(d, T);
     if (tv > clean) {  // block-uniform; the scan empties what a row used
-      for (uint32_t i = clean + threadIdx.x; i < tv; i += kThreads) {
+      for (uint32_t i = clean + threadIdx.x; i < tv; i += NT) {
         keys[i] = kEmptyKey;
         vals[i] = 0.0;
       }
@@ -967,7 +974,7 @@ __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int c
     bool hot_seen = false;
     uint32_t slots[(MAXW + 1) / 2] = {};
     uint32_t owned;
-    insert_block_range<MAXW, RULE>(L, s, 0, d, v, cv, keys, vals, tv - 1, own, hot,
+    insert_block_range<MAXW, RULE, NT>(L, s, 0, d, v, cv, keys, vals, tv - 1, own, hot,
                                    hot_seen, slots, owned);
     // every warp adds its share of the own community's weight to that
     // community's slot (FP64 sums of FP32 weights are exact in any order),
@@ -995,7 +1002,7 @@ __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int c
     if (threadIdx.x == 0) {
       K b = red_best[0];
       double o = red_own[0];
-      for (int i = 1; i < kWarps; i++) {
+      for (int i = 1; i < NT / 32; i++) {
         b = best_max(b, red_best[i]);
         if (RULE == LV_RULE_CUDA_I) o += red_own[i];
       }
@@ -2154,6 +2161,8 @@ __global__ void __launch_bounds__(kThreads, kLoopPerSM)
   }
 }
 
+#include "small_run.cuh"
+
 // ---------------------------------------------------------------------------
 // Small helpers
 // ---------------------------------------------------------------------------
@@ -2256,7 +2265,7 @@ __global__ void bucket_ids_kernel(const uint64_t* off, uint32_t n, uint8_t* out)
 // 4-byte gather of the neighbour's community each.  A warp takes 32
 // consecutive rows as one flat range of entries, so every load but the
 // gather is coalesced (a thread per row read a sector per entry, and each
-// row twice: 530 -> 77 us for 1 M vertices and 14 M entries).  Rows above
+// row twice: 530 -> 207 us for 1 M vertices and 14 M entries).  Rows above
 // kPartLong entries go to a list of (row, chunk) pairs that the whole grid
 // shares afterwards.  acc: [0] intra, [1] squared totals, [2] all weight,
 // [3] vertices with a community id >= n (skipped: the caller refuses the
@@ -2694,6 +2703,67 @@ cudaError_t launch_level_loop(const PassDesc* D, int mode, cudaStream_t st) {
     case 1: return launch_loop_impl<1>(D, st);
     case 2: return launch_loop_impl<2>(D, st);
     case 3: return launch_loop_impl<3>(D, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+template <int MODE>
+static cudaLaunchConfig_t small_run_config(cudaLaunchAttribute* at, unsigned ctas,
+                                           cudaStream_t st) {
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(ctas);
+  lc.blockDim = dim3(kSmallThreads);
+  lc.dynamicSmemBytes = kSmallSmem;
+  lc.stream = st;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  return lc;
+}
+
+// Largest cluster the device can run the small-run kernel with (16, 8, or 0:
+// none), once per process.
+template <int MODE>
+static int small_run_cluster() {
+  static const int size = [] {
+    const void* f = (const void*)small_run_kernel<MODE>;
+    int found = 0;
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kSmallSmem) == cudaSuccess &&
+        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+            cudaSuccess) {
+      for (int c = kSmallCtas; c >= 8 && !found; c /= 2) {
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t lc = small_run_config<MODE>(at, (unsigned)c, nullptr);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, f, &lc) == cudaSuccess && n > 0) found = c;
+      }
+    }
+    cudaGetLastError();
+    return found;
+  }();
+  return size;
+}
+
+template <int MODE>
+static cudaError_t launch_small_run_impl(const SmallRunArgs& A, bool one, cudaStream_t st) {
+  const int most = small_run_cluster<MODE>();
+  if (!most) return cudaErrorNotSupported;
+  cudaLaunchAttribute at[1];
+  const cudaLaunchConfig_t lc = small_run_config<MODE>(at, one ? 1u : (unsigned)most, st);
+  count_launches(1);
+  return cudaLaunchKernelEx(&lc, small_run_kernel<MODE>, A,
+                            one ? kSmallOneMaxN : kSmallMaxN);
+}
+
+cudaError_t launch_small_run(const SmallRunArgs& A, int mode, bool one, cudaStream_t st) {
+  switch (mode) {
+    case 0: return launch_small_run_impl<0>(A, one, st);
+    case 1: return launch_small_run_impl<1>(A, one, st);
+    case 2: return launch_small_run_impl<2>(A, one, st);
+    case 3: return launch_small_run_impl<3>(A, one, st);
     default: return cudaErrorInvalidValue;
   }
 }
