@@ -498,6 +498,7 @@ __device__ __forceinline__ void record_decision(const PassDesc* __restrict__ D,
 template <int G, int MODE, int NT = kThreads>
 __device__ __forceinline__ void small_body(const PassDesc* __restrict__ D, int cls,
                                            uint32_t bid, uint32_t nblk, double (*sums)[32],
+                                           uint32_t (*lead_sm)[64],
                                            const StepIO io = StepIO{}) {
   constexpr int RULE = ModeOf<MODE>::kRule, PREC = ModeOf<MODE>::kPrec;
   using K = typename BestOf<PREC>::T;
@@ -537,8 +538,6 @@ __device__ __forceinline__ void small_body(const PassDesc* __restrict__ D, int c
       u = L.col[s + gl];
       wt = L.w[s + gl];
       cu = L.comm[u];
-      szc = candidate_size(L, g, cu);  // the candidate's data, read before the grouping
-      ac = L.tot[cu];
     }
     // the own community's entries are summed with shuffles (its lowest
     // lane holds the sum); the others through one shared slot per distinct
@@ -549,17 +548,38 @@ __device__ __forceinline__ void small_body(const PassDesc* __restrict__ D, int c
     const unsigned gmask = (G == 32) ? kFull : (((1u << G) - 1u) << (lane & ~(G - 1)));
     const unsigned hmask = __ballot_sync(kFull, is_hot) & gmask;
     const int hot_leader = hmask ? __ffs(hmask) - 1 : -1;
-    // leader of an entry: the group's lowest lane holding the same community
+    // leader of an entry: one lane of the group holding the same community
     const uint32_t gbase = lane & ~(G - 1);
-    const uint32_t mykey = ins ? cu : kEmptyKey;
-    uint32_t first = gl;
+    int leader = lane;
+    if constexpr (G >= 16) {
+      // every lane writes its number to its community's slot (2 G slots per
+      // group); the lanes that read back a lane of their own community have
+      // their leader, the others try again without them.  Two or three
+      // rounds, where G - 1 shuffles took 2,600 cycles a vertex at G = 32.
+      uint32_t* slot = &lead_sm[wib][(2 * gbase) + ((cu * 2654435761u) >> (G == 32 ? 26 : 27))];
+      bool pending = ins;
+      while (__any_sync(kFull, pending)) {
+        if (pending) *slot = lane;
+        __syncwarp();
+        const int w = pending ? (int)*slot : lane;
+        const uint32_t wk = __shfl_sync(kFull, cu, w);
+        if (pending && wk == cu) {
+          leader = w;
+          pending = false;
+        }
+        __syncwarp();
+      }
+    } else {
+      const uint32_t mykey = ins ? cu : kEmptyKey;
+      uint32_t first = gl;
 #pragma unroll
-    for (int o = 1; o < G; o++) {
-      const uint32_t src = (gl + o) & (G - 1);
-      const uint32_t ok = __shfl_sync(kFull, mykey, gbase | src);
-      if (ins && ok == cu && src < first) first = src;
+      for (int o = 1; o < G; o++) {
+        const uint32_t src = (gl + o) & (G - 1);
+        const uint32_t ok = __shfl_sync(kFull, mykey, gbase | src);
+        if (ins && ok == cu && src < first) first = src;
+      }
+      leader = (int)(gbase | first);
     }
-    const int leader = (int)(gbase | first);
     sums[wib][lane] = (lane == hot_leader) ? hv : 0.0;
     __syncwarp();
     if (ins) atomicAdd(&sums[wib][leader], (double)wt);
@@ -567,6 +587,10 @@ __device__ __forceinline__ void small_body(const PassDesc* __restrict__ D, int c
     if (RULE == LV_RULE_CUDA_I && is_hot && u != v) own = (double)wt;
     __syncwarp();
     K best{};
+    if ((ins && leader == lane) || lane == hot_leader) {
+      szc = candidate_size(L, g, cu);
+      ac = L.tot[cu];
+    }
     if ((ins && leader == lane) || lane == hot_leader)
       best = candidate_loaded<PREC>(g, cu, sums[wib][lane], szc, ac);
     best = group_max<G>(best);
@@ -581,7 +605,8 @@ template <int G, int MODE>
 __global__ void __launch_bounds__(kThreads, kSmallPerSM)
     move_small_kernel(const PassDesc* __restrict__ D, int cls, StepIO io) {
   __shared__ double sums[kWarps][32];
-  small_body<G, MODE>(D, cls, blockIdx.x, gridDim.x, sums, io);
+  __shared__ uint32_t lead_sm[kWarps][64];
+  small_body<G, MODE>(D, cls, blockIdx.x, gridDim.x, sums, lead_sm, io);
 }
 
 // Best candidate among the taken slots of the first tv slots (nthr
@@ -1914,7 +1939,7 @@ constexpr int kLoopPerSM = 4;
 constexpr int kLoopSmem = kBlockTabSmem;
 static_assert(kLoopSmem >= kWarps * 512 * kSlotBytes && kLoopSmem >= kHubPartSmem &&
                   kLoopSmem >= (int)(kHubMaxParts * sizeof(uint32_t)) &&
-                  kLoopSmem >= (int)(kWarps * 32 * sizeof(double)),
+                  kLoopSmem >= (int)(kWarps * (32 * sizeof(double) + 64 * sizeof(uint32_t))),
               "every phase's shared memory fits the arena");
 // A barrier wait longer than this is a fault (a phase of the largest graphs
 // lasts milliseconds): the block sets the abort flag and the kernel ends.
@@ -1972,7 +1997,8 @@ __device__ __forceinline__ bool grid_barrier(LevelLoopState* S, uint32_t nblk,
 template <int G, int MODE>
 __device__ __noinline__ void small_phase(const PassDesc* __restrict__ D, int cls, uint32_t bid,
                                          uint32_t nblk, unsigned char* smem, StepIO io) {
-  small_body<G, MODE>(D, cls, bid, nblk, reinterpret_cast<double(*)[32]>(smem), io);
+  small_body<G, MODE>(D, cls, bid, nblk, reinterpret_cast<double(*)[32]>(smem),
+                      reinterpret_cast<uint32_t(*)[64]>(smem + kWarps * 32 * sizeof(double)), io);
 }
 template <int T, int MAXW, int MODE>
 __device__ __noinline__ void warp_phase(const PassDesc* __restrict__ D, int cls, uint32_t bid,

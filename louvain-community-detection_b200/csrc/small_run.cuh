@@ -250,7 +250,9 @@ __device__ __noinline__ void small_rows(const LevelView& L, const SmallMem& M, b
 
 template <int G, int MODE>
 __device__ __noinline__ void small_lanes(const PassDesc* D, int cls, unsigned char* smem) {
-  small_body<G, MODE, kSmallThreads>(D, cls, 0, 1, reinterpret_cast<double(*)[32]>(smem));
+  small_body<G, MODE, kSmallThreads>(
+      D, cls, 0, 1, reinterpret_cast<double(*)[32]>(smem),
+      reinterpret_cast<uint32_t(*)[64]>(smem + kSmallWarps * 32 * sizeof(double)));
 }
 template <int T, int MAXW, int MODE>
 __device__ __noinline__ void small_warp(const PassDesc* D, int cls, unsigned char* smem,
