@@ -967,16 +967,17 @@ lv_status issue_pass(lv_engine* E, const PassControl* ctl);
 constexpr uint64_t kIncrementalMinEntries = 1ull << 23;
 
 // The kernel of bucket b on this level: the tuned (or default) variant,
-// except that a warp-per-vertex bucket with no more vertices than the block
-// kernel has resident blocks gives each vertex a whole block -- there the
-// launch lasts as long as one vertex's chain, which a block shortens
-// (single graph; a union keeps its tuning).
+// except that a warp-per-vertex bucket with at most twice as many vertices as
+// teams of four warps are resident runs a team per vertex -- there the launch
+// lasts as long as one vertex's chain, which the team shortens (bench
+// power-law graph: 5.59 -> 5.54 ms, LFR 100 K 4.06 -> 4.00 ms; at 4,868
+// vertices the banded matrix's level 0 went from 0.48 to 0.57 ms).  Single
+// graph; a union keeps its tuning.
 uint8_t effective_variant(const lv_engine* E, int b) {
   const uint8_t v = E->tune[b];
-  if (E->batch || b < 1 || b > 6) return v;
-  if (v != KV_WARP128 && v != KV_WARP512) return v;
+  if (E->batch || b < 1 || b > 6 || v != KV_WARP128) return v;
   const uint32_t cnt = E->plan.cls_start[b + 1] - E->plan.cls_start[b];
-  return (cnt > 0 && cnt <= move_block_resident()) ? (uint8_t)KV_BLOCK : v;
+  return (cnt > 0 && cnt <= 2 * move_team_resident()) ? (uint8_t)KV_WARP512 : v;
 }
 
 // Writes the current level into the device pass descriptor (every pass
@@ -2124,18 +2125,22 @@ constexpr uint64_t kSmallFirstEntries = 12288;
 constexpr uint64_t kSmallLaterEntries = 32768;
 constexpr uint64_t kSmallOneEntries = 1536;
 constexpr uint32_t kSmallOneVertices = 64;
+// A refused launch costs a host wait, 30 us: a contracted level whose entries
+// are not known yet is offered only when the level before had at most this
+// many (contractions of late levels shrink the entries four- to tenfold).
+constexpr uint64_t kSmallPrevEntries = 1ull << 18;
 
 static uint64_t small_max_entries(const lv_engine* E) {
   return E->levels.empty() ? kSmallFirstEntries : kSmallLaterEntries;
 }
 
 // A level the small-run kernel may take: the default single-graph path, not
-// set up yet.  Its entry count may still be on the device (agg_pending): the
-// kernel then refuses a level with too many.
+// set up yet.  Its entry count may still be on the device (agg_pending; E->e
+// is the level before's then): the kernel refuses a level with too many.
 static bool small_eligible(const lv_engine* E) {
   return E->cfg.use_graphs && !E->profiling && !E->batch && !use_level_kernel(E) &&
          !E->cfg.contract_sort && !E->cfg.apply_launch && !E->level_ready && !E->small_off &&
-         E->n > 0 && E->n <= kSmallMaxN && (E->agg_pending || E->e <= small_max_entries(E));
+         E->n > 0 && E->n <= kSmallMaxN && E->e <= (E->agg_pending ? kSmallPrevEntries : small_max_entries(E));
 }
 
 // Runs the engine's level (with move_only its passes, else every level to the

@@ -428,8 +428,8 @@ DispatchArgs dispatch_args(const uint32_t* order, const DispatchPlan& P, const u
 // order[].
 // act_cnt: as for launch_modularity (null: whole classes).
 // Move kernel variants a bucket can run on: G-lane groups (one entry per
-// lane, degree <= G), a warp with a 128- or 512-slot shared table, a block
-// with a 4096-slot table.  All give the same proposals; they differ in how
+// lane, degree <= G), a warp with a 128-slot shared table, a block of four
+// warps with a 512-slot one, a block of eight with a 4096-slot one.  All give the same proposals; they differ in how
 // the work maps onto the SMs, which the autotuner measures.
 enum MoveVariant : uint8_t {
   KV_SMALL4 = 0,
@@ -488,8 +488,8 @@ cudaError_t launch_modularity_of(const LevelView& L, const uint32_t* part,
 cudaError_t launch_bucket_ids(const uint64_t* off, uint32_t n, uint8_t* out,
                               cudaStream_t st);
 unsigned dispatch_grid(const DispatchPlan& P);
-// Blocks of the block-per-vertex move kernel resident on the device at once.
-unsigned move_block_resident();
+// Blocks of the four-warps-per-vertex move kernel resident on the device at once.
+unsigned move_team_resident();
 unsigned sm_count_cached();
 // Opts kernels with more than 48 KB of shared memory in (once per device).
 cudaError_t configure_kernels();

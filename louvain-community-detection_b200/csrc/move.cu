@@ -32,9 +32,9 @@
 //     equal communities in a group are found with G - 1 shuffles, no hash
 //     table at all.  (__match_any_sync costs about one step per distinct
 //     value in the warp, and at level 0 all 32 values are distinct.)
-//     32 < deg <= 319: one warp per vertex, open-addressing table in shared
-//     memory.  319 < deg <= 2048: one block per vertex, 4096-slot shared
-//     table.  deg > 2048: one block per (vertex, hash partition of its
+//     32 < deg <= 84: one warp per vertex, open-addressing table in shared
+//     memory.  deg <= 319: a block of four warps per vertex, 512 slots.
+//     319 < deg <= 2048: a block of eight, 4096 slots.  deg > 2048: one block per (vertex, hash partition of its
 //     neighbour communities), 4096-slot shared table, the partitions' best
 //     candidates merged with one 64-bit atomicMax each -- no global hash
 //     table, whatever the degree.  Shared tables are self-cleaning: a row
@@ -58,7 +58,6 @@ constexpr int kWarps = kThreads / 32;
 // (a grid above residency would run a partial second wave of blocks).
 constexpr int kSmallPerSM = 8;     // 32 registers
 constexpr int kWarp128PerSM = 5;   // 48 registers, 12 KB tables
-constexpr int kWarp512PerSM = 4;   // 64 registers, 48 KB tables
 constexpr int kBlockPerSM = 3;     // 80 registers, 48 KB table
 constexpr int kSplitPerSM = 4;
 constexpr int kMergePerSM = 3;     // 80 registers (4 per SM at 64: 9% slower on R-MAT 24)
@@ -867,7 +866,7 @@ __device__ __forceinline__ void warp_body(const PassDesc* __restrict__ D, int cl
 }
 
 template <int T, int MAXW, int MODE>
-__global__ void __launch_bounds__(kThreads, T == 128 ? kWarp128PerSM : kWarp512PerSM)
+__global__ void __launch_bounds__(kThreads, kWarp128PerSM)
     move_warp_kernel(const PassDesc* __restrict__ D, int cls, StepIO io) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   warp_body<T, MAXW, MODE>(D, cls, blockIdx.x, gridDim.x, smem_raw, io);
@@ -954,7 +953,8 @@ __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t 
   }
 }
 
-template <int MODE, int NT = kThreads>
+// A block of NT threads per vertex of at most MAXDEG entries, T-slot table.
+template <int MODE, int NT = kThreads, int T = kHubSmemSlots, int MAXDEG = (int)kHubSmemMaxDeg>
 __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int cls, uint32_t bid,
                                            uint32_t nblk, unsigned char* smem_raw,
                                            typename BestOf<ModeOf<MODE>::kPrec>::T* red_best,
@@ -962,18 +962,19 @@ __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int c
   constexpr int RULE = ModeOf<MODE>::kRule, PREC = ModeOf<MODE>::kPrec;
   using K = typename BestOf<PREC>::T;
   const LevelView L = step_view(D, io);
-  reapply_prev_step(D, io, bid, nblk);
-  record_pass_start(D, L, io, bid, nblk);
   const uint32_t s0 = D->A.P.cls_start[cls];
   const uint32_t* __restrict__ verts = D->A.order + s0;
   uint32_t* __restrict__ prop = D->prop + s0;
   const uint32_t count = D->act_cnt ? D->act_cnt[cls] : D->A.P.cls_start[cls + 1] - s0;
-  constexpr int T = kHubSmemSlots;
-  constexpr int MAXW = (int)(kHubSmemMaxDeg / NT);
+  constexpr int MAXW = (MAXDEG + NT - 1) / NT;
   double* vals = reinterpret_cast<double*>(smem_raw);
   uint32_t* keys = reinterpret_cast<uint32_t*>(smem_raw + sizeof(double) * T);
   uint32_t clean = 0;  // leading table slots known to be empty
+  // the first vertex's id, row and community are on their way while the
+  // previous step's moves are applied (to the other copy)
   VertexRow nxt = fetch_vertex(L, verts, bid, count);
+  reapply_prev_step(D, io, bid, nblk);
+  record_pass_start(D, L, io, bid, nblk);
   for (uint32_t vidx = bid; vidx < count; vidx += nblk) {
     const uint32_t v = nxt.v;
     const uint64_t s = nxt.s;
@@ -1049,6 +1050,26 @@ __global__ void __launch_bounds__(kThreads, kBlockPerSM)
   __shared__ typename BestOf<ModeOf<MODE>::kPrec>::T red_best[kWarps];
   __shared__ double red_own[kWarps];
   block_body<MODE>(D, cls, blockIdx.x, gridDim.x, smem_raw, red_best, red_own, io);
+}
+
+// deg <= 319 (KV_WARP512): a block of four warps per vertex, 512-slot table.
+// What bounds it is one vertex's chain of L2 round trips and table rounds: a
+// warp per vertex needed ten insert rounds and sixteen table slots a lane for
+// such a row, 40 us a launch however few vertices (bench power-law graph, 1,361
+// vertices); four warps take a quarter of the rounds, 14.6 us.  On levels with
+// many such vertices the time is the same or less (LFR 1 M: 101 -> 54 us,
+// R-MAT 24: 1,844 -> 1,711 us a launch).
+constexpr int kTeamThreads = 128;
+constexpr int kTeamSlots = 512;
+constexpr int kTeamPerSM = 10;  // 48 registers
+template <int MODE>
+__global__ void __launch_bounds__(kTeamThreads, kTeamPerSM)
+    move_team_kernel(const PassDesc* __restrict__ D, int cls, StepIO io) {
+  __shared__ __align__(16) unsigned char smem_raw[kTeamSlots * kSlotBytes];
+  __shared__ typename BestOf<ModeOf<MODE>::kPrec>::T red_best[kTeamThreads / 32];
+  __shared__ double red_own[kTeamThreads / 32];
+  block_body<MODE, kTeamThreads, kTeamSlots, 319>(D, cls, blockIdx.x, gridDim.x, smem_raw,
+                                                  red_best, red_own, io);
 }
 
 // deg > 2048 (hubs).  The neighbour communities of a hub are split into P
@@ -2512,12 +2533,8 @@ unsigned sm_count_cached() {
 
 template <int MODE>
 static cudaError_t configure_mode() {
-  const int warp512 = kWarps * 512 * kSlotBytes;
-  cudaError_t e = cudaFuncSetAttribute(move_warp_kernel<512, 10, MODE>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, warp512);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(move_block_kernel<MODE>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, kBlockTabSmem);
+  cudaError_t e = cudaFuncSetAttribute(move_block_kernel<MODE>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kBlockTabSmem);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(hub_merge_kernel<MODE>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, kHubPartSmem);
@@ -2618,7 +2635,7 @@ cudaError_t launch_modularity_pass(const PassDesc* D, const PassControl* ctl, cu
 }
 
 unsigned pass_dispatch_grid() { return sm_count() * kModPerSM; }
-unsigned move_block_resident() { return sm_count() * kBlockPerSM; }
+unsigned move_team_resident() { return sm_count() * kTeamPerSM; }
 
 // One launch of a move kernel variant over class `cls`.
 template <int MODE>
@@ -2643,12 +2660,10 @@ static void launch_variant(int kv, const PassDesc* D, int cls, cudaStream_t st, 
                                                        kWarps * T * kSlotBytes, st>>>(D, cls, io));
       break;
     }
-    case KV_WARP512: {
-      constexpr int T = 512;
-      (count_launches(1), move_warp_kernel<T, 10, MODE><<<sm_count() * kWarp512PerSM, kThreads,
-                                                        kWarps * T * kSlotBytes, st>>>(D, cls, io));
+    case KV_WARP512:
+      (count_launches(1), move_team_kernel<MODE><<<sm_count() * kTeamPerSM, kTeamThreads, 0, st>>>(
+          D, cls, io));
       break;
-    }
     default:  // KV_BLOCK: shared table, one block per vertex
       (count_launches(1), move_block_kernel<MODE><<<sm_count() * kBlockPerSM, kThreads,
                                                    kBlockTabSmem, st>>>(D, cls, io));
