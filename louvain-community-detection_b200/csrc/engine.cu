@@ -416,7 +416,7 @@ struct lv_engine {
   size_t act_order_cap = 0;
   uint32_t* act_cnt = nullptr;  // [16]
   uint32_t* cg = nullptr;       // [kMoveClasses * (graph cap + 1)]
-  uint32_t* cg_new = nullptr;
+  uint32_t* cg_new = nullptr;   // then the entry chunks' starts (UnionChunks)
 
   // all passes of a level as one graph (WHILE node), one per key (form,
   // rule, tuning, which kernel classes are non-empty), most recent last
@@ -860,9 +860,9 @@ lv_status prepare_level(lv_engine* E, bool sync_scalars = true) {
   u += P.hub_blocks;
   P.blk_start[9] = u;
   P.total_blocks = u;
-  // partials: hub accumulators + 2 per dispatch block
+  // partials: hub accumulators + 3 per dispatch block
   const size_t need_partials =
-      hc + 2 * (size_t)std::max(dispatch_grid(P), pass_dispatch_grid()) + 16;
+      hc + 3 * (size_t)std::max(dispatch_grid(P), pass_dispatch_grid()) + 16;
   if (need_partials > E->partials_cap) {
     E->partials_cap = 0;
     dfree(E->partials);
@@ -935,21 +935,18 @@ lv_status prepare_level(lv_engine* E, bool sync_scalars = true) {
     CU(cudaMemcpyAsync(E->class_deg, E->d_class_deg, kClasses * sizeof(uint64_t),
                        cudaMemcpyDeviceToHost, st));
   }
-  // row sums, singleton state, m; then Q of the singleton partition.  A
-  // single graph's level init also writes the row of every entry, for the
-  // pass loop's modularity sweep (kept in the contraction's column scratch
-  // until the level ends), and the incremental sweep's pass-start
-  // communities (singletons)
+  // row sums, singleton state, m, Q of the singleton partition and the row of
+  // every entry, for the pass loop's modularity sweep (kept in the
+  // contraction's column scratch until the level ends); a single graph also
+  // the incremental sweep's pass-start communities (singletons)
   const LevelView L = E->view();
   const double Vd = (double)n, Ed = (double)E->e;
   cudaEvent_t t0 = prof_begin(E);
-  CU(launch_level_init(L, E->order, P, hc ? E->hub_map : nullptr, E->partials,
-                       E->batch ? nullptr : E->cb.tcol, E->batch ? nullptr : E->comm_start,
-                       st));
-  prof_end(E, t0, K_LEVEL_INIT, Ed * 4.0 + Vd * 32.0);
-  t0 = prof_begin(E);
-  CU(launch_modularity(L, E->order, P, hc ? E->hub_map : nullptr, E->partials, st));
-  prof_end(E, t0, K_MODULARITY, Ed * 12.0 + Vd * 24.0);
+  CU(launch_level_init(L, E->order, P, hc ? E->hub_map : nullptr, E->partials, E->cb.tcol,
+                       E->batch ? nullptr : E->comm_start, st));
+  prof_end(E, t0, K_LEVEL_INIT, Ed * 8.0 + Vd * 32.0);
+  // the level's first evaluation of Q is part of that launch: counted, no time
+  if (E->profiling) E->kst[K_MODULARITY].launches++;
   if (sync_scalars) {  // else the level graph's own synchronisation reads them
     CU(cudaMemcpyAsync(E->sc_host, E->sc, sizeof(LevelScalars),
                        cudaMemcpyDeviceToHost, st));
@@ -987,7 +984,6 @@ lv_status upload_desc(lv_engine* E, float min_gain) {
   d.L = E->view();
   const uint32_t* ord = E->batch ? E->act_order : E->order;
   d.A = dispatch_args(ord, E->plan, E->plan.hub_count ? E->hub_map : nullptr, E->partials);
-  d.A.act_cnt = E->batch ? E->act_cnt : nullptr;
   d.prop = E->prop;
   d.full_order = E->order;
   d.H = E->hub;
@@ -996,9 +992,11 @@ lv_status upload_desc(lv_engine* E, float min_gain) {
   d.cg = E->cg;
   d.cg_new = E->cg_new;
   d.n_graphs = E->batch ? E->n_graphs : 0u;
-  // single graph: row ids built by prepare_level in the contraction's
-  // column scratch, which is idle until the level's pass loop ends
-  d.rowid = E->batch ? nullptr : E->cb.tcol;
+  d.chunk_start = E->batch ? E->cg_new + (size_t)kMoveClasses * (E->n_graphs + 1) : nullptr;
+  d.goff = E->batch ? E->goff_dev : nullptr;
+  // row ids built by prepare_level in the contraction's column scratch, which
+  // is idle until the level's pass loop ends
+  d.rowid = E->cb.tcol;
   d.nnz = E->e;
   d.min_gain = (double)min_gain;
   d.max_passes = E->cfg.max_passes;
@@ -1340,7 +1338,7 @@ lv_status batch_alloc(lv_engine* E, uint32_t G) {
   if (E->gs_host) cudaFreeHost(E->gs_host);
   E->gs_host = nullptr;
   CU(dalloc(&E->cg, (size_t)kMoveClasses * (G + 1)));
-  CU(dalloc(&E->cg_new, (size_t)kMoveClasses * (G + 1)));
+  CU(dalloc(&E->cg_new, (size_t)(kMoveClasses + 1) * (G + 1)));
   CU(dalloc(&E->act_cnt, 16));
   CU(dalloc(&E->gs, G));
   CU(dalloc(&E->goff_dev, (size_t)G + 1));

@@ -246,18 +246,15 @@ cudaError_t partition_by_size4(const uint64_t* sizes, uint32_t n_upper,
 // ---------------------------------------------------------------------------
 // move.cu
 // ---------------------------------------------------------------------------
-// Row sums k_v, singleton state (comm=id, sizes 1, totals k) and m; with
-// rowid the row of every entry, with comm_start comm_start[v] = v.
+// Row sums k_v, singleton state (comm=id, sizes 1, totals k), m and the
+// modularity of the singleton partition; with rowid the row of every entry,
+// with comm_start comm_start[v] = v.
 cudaError_t launch_level_init(const LevelView& L, const uint32_t* order,
                               const DispatchPlan& P, const uint32_t* hub_map,
                               double* partials, uint32_t* rowid, uint32_t* comm_start,
                               cudaStream_t st);
-// Modularity of the current state into sc->q (FP64, deterministic).  With
-// ctl->enabled the last block also applies the pass stop rule and sets the
-// graph condition.
-// With act_cnt (batched form) classes 1..7 of `order` are the compacted
-// active lists and act_cnt[c] their device-side lengths; every graph's
-// modularity then comes from its own vertices' rows and totals.
+// Modularity of a single graph's current state into sc->q (FP64,
+// deterministic).
 cudaError_t launch_modularity(const LevelView& L, const uint32_t* order,
                               const DispatchPlan& P, const uint32_t* hub_map,
                               double* partials, cudaStream_t st);
@@ -306,8 +303,19 @@ struct DispatchArgs {
   const uint32_t* hub_blk_vertex;
   const uint32_t* hub_blk_chunk;
   double* hub_acc;
-  double* partials;         // [2 * gridDim.x]
-  const uint32_t* act_cnt;  // batched form: active lengths of classes 1..7
+  double* partials;         // [3 * gridDim.x]
+};
+
+// Batched form: entries per chunk of the modularity sweep, its inputs (first
+// chunk of every active graph, the graphs' vertex offsets, the number of
+// chunks), and where the compaction leaves that number beside the classes'
+// active lengths.
+constexpr uint32_t kUnionChunk = 4096;
+constexpr int kUnionTotal = 9;
+struct UnionChunks {
+  const uint32_t* start = nullptr;
+  const uint32_t* goff = nullptr;
+  const uint32_t* total = nullptr;
 };
 
 // Everything a pass's kernels need about the current level, in device
@@ -344,8 +352,10 @@ struct PassDesc {
   const uint32_t* cg;
   uint32_t* cg_new;
   uint32_t n_graphs;
-  // single graph: the row of every entry (the modularity sweep runs over
-  // the entries, not the class lists); nullptr in the batched form
+  uint32_t* chunk_start;  // [n_graphs + 1] UnionChunks
+  const uint32_t* goff;
+  // the row of every entry (the modularity sweep runs over the entries, not
+  // the class lists)
   const uint32_t* rowid;
   uint64_t nnz;
   // device-side pass loop
@@ -426,7 +436,6 @@ DispatchArgs dispatch_args(const uint32_t* order, const DispatchPlan& P, const u
 // Proposals for the vertices of kernel class c (1..8; bucket 7 is classes 7
 // and 8, both launched before its apply).  proposal[] is parallel to
 // order[].
-// act_cnt: as for launch_modularity (null: whole classes).
 // Move kernel variants a bucket can run on: G-lane groups (one entry per
 // lane, degree <= G), a warp with a 128-slot shared table, a block of four
 // warps with a 512-slot one, a block of eight with a 4096-slot one.  All give the same proposals; they differ in how

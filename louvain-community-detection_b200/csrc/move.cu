@@ -269,27 +269,7 @@ __device__ __forceinline__ double group_sum(double x) {
   return x;
 }
 
-// Batched form: adds every lane's val into gs[key].*field with one atomic
-// per run of equal keys.  Called by all 32 lanes; keys must be
-// non-decreasing across the lanes (vertex ids ascend within a class order,
-// and graphs own contiguous id ranges), a lane without a value passes
-// kNoGraph.  A segmented suffix sum leaves each run's total in its first
-// lane.
 constexpr uint32_t kNoGraph = 0xFFFFFFFFu;
-using GraphField = double GraphState::*;
-__device__ __forceinline__ void warp_graph_add(GraphState* gs, GraphField field, uint32_t key,
-                                               double val) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const double ov = __shfl_down_sync(kFull, val, o);
-    const uint32_t ok = __shfl_down_sync(kFull, key, o);
-    if (lane + o < 32 && ok == key) val += ov;
-  }
-  const uint32_t pk = __shfl_up_sync(kFull, key, 1);
-  if (key != kNoGraph && (lane == 0 || pk != key) && val != 0.0)
-    atomicAdd(&(gs[key].*field), val);
-}
 
 // Open addressing with linear probing.  Probe counts are bounded by the
 // table size; a full table (impossible while a table holds more slots than
@@ -1378,53 +1358,75 @@ __global__ void __launch_bounds__(kThreads, kSweepPerSM)
 // ---------------------------------------------------------------------------
 // Class-dispatch row reductions (row sums at level start, modularity sweep)
 // ---------------------------------------------------------------------------
-// Row sum: k_v = (float) sum_j w_vj.  vertex() returns the vertex's share
-// of its graph's accumulator (batched form).
+// Row sums k_v = (float) sum_j w_vj with what the singleton partition's
+// modularity needs: the self-loops' weight and the squared totals.  Batched
+// form: a lane keeps the sums of the graph whose rows it works on and adds
+// them to the graph when it meets another's (a block's units of a class are
+// consecutive, and graphs are runs of every class list).
 struct RowSumOp {
-  static constexpr GraphField kField = &GraphState::m_acc;
-  static constexpr bool kAsq = false;
+  double m = 0.0, self = 0.0, asq = 0.0;
+  uint32_t graph = kNoGraph;
   __device__ bool row(const LevelView&, uint32_t) const { return true; }
-  __device__ uint32_t ctx(const LevelView&, uint32_t) const { return 0; }
-  __device__ double edge(const LevelView&, uint32_t, uint32_t, float w) const {
+  __device__ uint32_t ctx(const LevelView& L, uint32_t v) {
+    if (L.gid) {
+      const uint32_t g = L.gid[v];
+      if (g != graph) {
+        flush(L);
+        graph = g;
+      }
+    }
+    return v;
+  }
+  __device__ double edge(const LevelView&, uint32_t v, uint32_t u, float w) {
+    if (u == v) self += (double)w;
     return (double)w;
   }
-  __device__ double vertex(const LevelView& L, uint32_t v, double sum,
-                           double& part) const {
+  __device__ void vertex(const LevelView& L, uint32_t v, double sum) {
     const float kf = (float)sum;
+    const double kd = (double)kf;
     L.k[v] = kf;
-    L.tot[v] = (double)kf;
-    if (L.tot_alt) L.tot_alt[v] = (double)kf;
-    part += (double)kf;
-    return (double)kf;
+    L.tot[v] = kd;
+    if (L.tot_alt) L.tot_alt[v] = kd;
+    m += kd;
+    asq += kd * kd;
   }
-  __device__ void hub(const LevelView&, const DispatchArgs& A, uint32_t hi, uint32_t,
-                      double sum, double&) const {
+  __device__ void hub(const LevelView&, const DispatchArgs& A, uint32_t hi, double sum) {
     atomicAdd(&A.hub_acc[hi], sum);
+  }
+  __device__ void flush(const LevelView& L) {
+    if (graph != kNoGraph) {
+      GraphState& s = L.gs[graph];
+      if (m != 0.0) atomicAdd(&s.m_acc, m);
+      if (self != 0.0) atomicAdd(&s.intra_acc, self);
+      if (asq != 0.0) atomicAdd(&s.asq_acc, asq);
+    }
+    m = self = asq = 0.0;
+  }
+  // Batched form, whole warps: one atomic per sum where the lanes agree.
+  __device__ void finish(const LevelView& L) {
+    if (!__all_sync(kFull, graph == __shfl_sync(kFull, graph, 0))) {
+      flush(L);
+      return;
+    }
+    m = group_sum<32>(m);
+    self = group_sum<32>(self);
+    asq = group_sum<32>(asq);
+    if ((threadIdx.x & 31) == 0) flush(L);
+    else m = self = asq = 0.0;
   }
 };
 
 // Intra-community weight: sum_j w_vj [comm(u) == comm(v)].
 struct IntraOp {
-  static constexpr GraphField kField = &GraphState::intra_acc;
-  // batched form: the vertex's community total squared (community ids are
-  // vertex ids), so an active graph's sum of a_c^2 comes with its rows
-  static constexpr bool kAsq = true;
+  double part = 0.0;
   __device__ bool row(const LevelView&, uint32_t) const { return true; }
-  __device__ uint32_t ctx(const LevelView& L, uint32_t v) const {
-    return L.comm[v];
-  }
-  __device__ double edge(const LevelView& L, uint32_t cv, uint32_t u,
-                         float w) const {
+  __device__ uint32_t ctx(const LevelView& L, uint32_t v) const { return L.comm[v]; }
+  __device__ double edge(const LevelView& L, uint32_t cv, uint32_t u, float w) const {
     return L.comm[u] == cv ? (double)w : 0.0;
   }
-  __device__ double vertex(const LevelView&, uint32_t, double sum, double& part) const {
+  __device__ void vertex(const LevelView&, uint32_t, double sum) { part += sum; }
+  __device__ void hub(const LevelView&, const DispatchArgs&, uint32_t, double sum) {
     part += sum;
-    return sum;
-  }
-  __device__ void hub(const LevelView& L, const DispatchArgs&, uint32_t, uint32_t v,
-                      double sum, double& part) const {
-    part += sum;
-    if (L.gid && sum != 0.0) atomicAdd(&L.gs[L.gid[v]].intra_acc, sum);
   }
 };
 
@@ -1437,8 +1439,7 @@ struct IntraOp {
 // weights are exact, so the updated sum equals a full sweep's.
 struct DeltaIntraOp {
   const uint32_t* cs;
-  static constexpr GraphField kField = &GraphState::intra_acc;
-  static constexpr bool kAsq = false;
+  double part = 0.0;
   __device__ bool row(const LevelView& L, uint32_t v) const { return cs[v] != L.comm[v]; }
   __device__ uint2 ctx(const LevelView& L, uint32_t v) const {
     return make_uint2(cs[v], L.comm[v]);
@@ -1450,41 +1451,19 @@ struct DeltaIntraOp {
     const double x = (csu != cu) ? (double)w : 2.0 * (double)w;
     return now ? x : -x;
   }
-  __device__ double vertex(const LevelView&, uint32_t, double sum, double& part) const {
-    part += sum;
-    return sum;
-  }
-  __device__ void hub(const LevelView&, const DispatchArgs&, uint32_t, uint32_t, double sum,
-                      double& part) const {
+  __device__ void vertex(const LevelView&, uint32_t, double sum) { part += sum; }
+  __device__ void hub(const LevelView&, const DispatchArgs&, uint32_t, double sum) {
     part += sum;
   }
 };
 
-__device__ __forceinline__ double sq(double a) { return a * a; }
-
-// Length of class cls's list: the active length in the batched form's
-// compacted lists, else the whole class.
 __device__ __forceinline__ uint32_t class_count(const DispatchArgs& A, int cls) {
-  return A.act_cnt ? A.act_cnt[cls] : A.P.cls_start[cls + 1] - A.P.cls_start[cls];
-}
-
-// Batched form, one lane for one vertex: its share of its graph's
-// accumulator (and its community total squared for the sweep).
-template <class Op>
-__device__ __forceinline__ void graph_add_one(const LevelView& L, uint32_t v, double share) {
-  GraphState& s = L.gs[L.gid[v]];
-  if (share != 0.0) atomicAdd(&(s.*Op::kField), share);
-  if (Op::kAsq) {
-    const double a = L.tot[v];
-    if (a != 0.0) atomicAdd(&s.asq_acc, a * a);
-  }
+  return A.P.cls_start[cls + 1] - A.P.cls_start[cls];
 }
 
 template <int G, class Op>
-__device__ __forceinline__ void unit_small(const LevelView& L,
-                                           const DispatchArgs& A, int cls,
-                                           uint32_t unit, const Op& op,
-                                           double& part) {
+__device__ __forceinline__ void unit_small(const LevelView& L, const DispatchArgs& A, int cls,
+                                           uint32_t unit, Op& op) {
   const int lane = threadIdx.x & 31, gl = lane & (G - 1);
   const uint32_t cnt = class_count(A, cls);
   const uint32_t idx = unit * (kThreads / G) + threadIdx.x / G;
@@ -1500,23 +1479,12 @@ __device__ __forceinline__ void unit_small(const LevelView& L,
     }
   }
   x = group_sum<G>(x);
-  double share = 0.0, a2 = 0.0;
-  if (idx < cnt && gl == 0) {
-    share = op.vertex(L, v, x, part);
-    if (Op::kAsq && L.gid) a2 = sq(L.tot[v]);
-  }
-  if (L.gid) {  // warp-uniform
-    const uint32_t key = idx < cnt ? L.gid[v] : kNoGraph;
-    warp_graph_add(L.gs, Op::kField, key, share);
-    if (Op::kAsq) warp_graph_add(L.gs, &GraphState::asq_acc, key, a2);
-  }
+  if (idx < cnt && gl == 0) op.vertex(L, v, x);
 }
 
 template <class Op>
-__device__ __forceinline__ void unit_warp(const LevelView& L,
-                                          const DispatchArgs& A, int cls,
-                                          uint32_t unit, const Op& op,
-                                          double& part) {
+__device__ __forceinline__ void unit_warp(const LevelView& L, const DispatchArgs& A, int cls,
+                                          uint32_t unit, Op& op) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t cnt = class_count(A, cls);
   const uint32_t idx = unit * kWarps + wib;
@@ -1529,17 +1497,12 @@ __device__ __forceinline__ void unit_warp(const LevelView& L,
   double x = 0.0;
   for (uint32_t j = lane; j < d; j += 32) x += op.edge(L, c, L.col[s + j], L.w[s + j]);
   x = group_sum<32>(x);
-  if (lane == 0) {
-    const double share = op.vertex(L, v, x, part);
-    if (L.gid) graph_add_one<Op>(L, v, share);
-  }
+  if (lane == 0) op.vertex(L, v, x);
 }
 
 template <class Op>
-__device__ __forceinline__ void unit_block(const LevelView& L,
-                                           const DispatchArgs& A,
-                                           uint32_t unit, const Op& op,
-                                           double& part, double* red) {
+__device__ __forceinline__ void unit_block(const LevelView& L, const DispatchArgs& A,
+                                           uint32_t unit, Op& op, double* red) {
   const uint32_t idx = unit;
   if (idx >= class_count(A, 7)) return;  // block-uniform
   const uint32_t v = A.order[A.P.cls_start[7] + idx];
@@ -1551,22 +1514,15 @@ __device__ __forceinline__ void unit_block(const LevelView& L,
   for (uint32_t j = threadIdx.x; j < d; j += kThreads)
     x += op.edge(L, c, L.col[s + j], L.w[s + j]);
   x = block_sum(x, red);
-  if (threadIdx.x == 0) {
-    const double share = op.vertex(L, v, x, part);
-    if (L.gid) graph_add_one<Op>(L, v, share);
-  }
+  if (threadIdx.x == 0) op.vertex(L, v, x);
 }
 
 template <class Op>
-__device__ __forceinline__ void unit_hub(const LevelView& L,
-                                         const DispatchArgs& A, uint32_t unit,
-                                         const Op& op, double& part,
-                                         double* red) {
+__device__ __forceinline__ void unit_hub(const LevelView& L, const DispatchArgs& A, uint32_t unit,
+                                         Op& op, double* red) {
   const uint32_t hb = unit;
   const uint32_t hi = A.hub_blk_vertex[hb], ch = A.hub_blk_chunk[hb];
   const uint32_t v = A.order[A.P.cls_start[8] + hi];
-  // batched pass loop: a finished graph's hubs need no sweep (block-uniform)
-  if (A.act_cnt && !L.gs[L.gid[v]].active) return;
   if (!op.row(L, v)) return;  // block-uniform
   const uint64_t s = L.off[v];
   const uint64_t d = L.off[v + 1] - s;
@@ -1576,25 +1532,23 @@ __device__ __forceinline__ void unit_hub(const LevelView& L,
   for (uint64_t j = lo + threadIdx.x; j < end; j += kThreads)
     x += op.edge(L, c, L.col[s + j], L.w[s + j]);
   x = block_sum(x, red);
-  if (threadIdx.x == 0) {
-    op.hub(L, A, hi, v, x, part);
-    if (Op::kAsq && L.gid && ch == 0 && L.tot[v] != 0.0)
-      atomicAdd(&L.gs[L.gid[v]].asq_acc, sq(L.tot[v]));
-  }
+  if (threadIdx.x == 0) op.hub(L, A, hi, x);
 }
 
 // Deterministic block reduction into partials, then the last block to
 // finish sums all partials in index order.
-__device__ __forceinline__ bool publish_and_check_last(double a, double b,
+__device__ __forceinline__ bool publish_and_check_last(double a, double b, double c,
                                                        const DispatchArgs& A,
                                                        LevelScalars* sc,
                                                        double* red) {
   __shared__ bool last;
   double ra = block_sum(a, red);
   double rb = block_sum(b, red);
+  double rc = block_sum(c, red);
   if (threadIdx.x == 0) {
     A.partials[blockIdx.x] = ra;
     A.partials[gridDim.x + blockIdx.x] = rb;
+    A.partials[2 * gridDim.x + blockIdx.x] = rc;
     __threadfence();
     const uint32_t t = atomicAdd(&sc->done_blocks, 1u);
     last = (t == gridDim.x - 1);
@@ -1604,54 +1558,34 @@ __device__ __forceinline__ bool publish_and_check_last(double a, double b,
   return last;
 }
 
-__device__ __forceinline__ void sum_partials(const DispatchArgs& A, double* red,
-                                             double& a, double& b) {
-  double x = 0.0, y = 0.0;
-  for (uint32_t i = threadIdx.x; i < gridDim.x; i += kThreads) {
-    x += __ldcg(&A.partials[i]);
-    y += __ldcg(&A.partials[gridDim.x + i]);
-  }
-  a = block_sum(x, red);
-  b = block_sum(y, red);
+__device__ __forceinline__ double sum_partials(const DispatchArgs& A, int which, double* red) {
+  double x = 0.0;
+  for (uint32_t i = threadIdx.x; i < gridDim.x; i += kThreads)
+    x += __ldcg(&A.partials[which * gridDim.x + i]);
+  return block_sum(x, red);
 }
 
-// Units of the class lists, grid-strided.  Every unit function gets its
-// unit's index within the class.  With act_cnt (batched pass loop) the
-// classes 1..7 hold only their active prefix, so the unit ranges are
-// derived from the device-side lengths and finished graphs cost nothing.
+// Units of the class lists: every class's units are split into one
+// consecutive range per block.
 template <class Op>
-__device__ __forceinline__ void dispatch_units(const LevelView& L,
-                                               const DispatchArgs& A,
-                                               const Op& op, double& part,
+__device__ __forceinline__ void dispatch_units(const LevelView& L, const DispatchArgs& A, Op& op,
                                                double* red) {
-  __shared__ uint32_t bs[kClasses + 1];
-  if (threadIdx.x == 0) {
-    if (A.act_cnt) {
-      bs[0] = bs[1] = 0u;
-      for (int c = 1; c <= kMoveClasses; c++) {
-        const uint32_t pu = class_per_unit(c);
-        bs[c + 1] = bs[c] + (A.act_cnt[c] + pu - 1) / pu;
+  for (int c = 1; c <= 8; c++) {
+    const uint64_t n = A.P.blk_start[c + 1] - A.P.blk_start[c];
+    // classes with few units start at different blocks
+    const uint32_t b = (blockIdx.x + (uint32_t)(c - 1) * (gridDim.x / 8)) % gridDim.x;
+    const uint32_t u0 = (uint32_t)(n * b / gridDim.x), u1 = (uint32_t)(n * (b + 1) / gridDim.x);
+    for (uint32_t u = u0; u < u1; u++) {
+      switch (c) {  // block-uniform
+        case 1: unit_small<4>(L, A, 1, u, op); break;
+        case 2: unit_small<8>(L, A, 2, u, op); break;
+        case 3: unit_small<16>(L, A, 3, u, op); break;
+        case 4: unit_small<32>(L, A, 4, u, op); break;
+        case 5:
+        case 6: unit_warp(L, A, c, u, op); break;
+        case 7: unit_block(L, A, u, op, red); break;
+        default: unit_hub(L, A, u, op, red); break;
       }
-      bs[9] = bs[8] + A.P.hub_blocks;
-    } else {
-      for (int c = 0; c <= kClasses; c++) bs[c] = A.P.blk_start[c];
-    }
-  }
-  __syncthreads();
-  const uint32_t total = bs[9];
-  for (uint32_t unit = blockIdx.x; unit < total; unit += gridDim.x) {
-    int cls = 8;
-    while (cls > 1 && unit < bs[cls]) cls--;
-    const uint32_t u = unit - bs[cls];
-    switch (cls) {  // block-uniform
-      case 1: unit_small<4>(L, A, 1, u, op, part); break;
-      case 2: unit_small<8>(L, A, 2, u, op, part); break;
-      case 3: unit_small<16>(L, A, 3, u, op, part); break;
-      case 4: unit_small<32>(L, A, 4, u, op, part); break;
-      case 5:
-      case 6: unit_warp(L, A, cls, u, op, part); break;
-      case 7: unit_block(L, A, u, op, part, red); break;
-      default: unit_hub(L, A, u, op, part, red); break;
     }
   }
 }
@@ -1660,8 +1594,9 @@ __global__ void __launch_bounds__(kThreads)
     level_init_kernel(LevelView L, DispatchArgs A, uint32_t* __restrict__ rowid,
                       uint32_t* __restrict__ comm_start) {
   __shared__ double red[kWarps];
-  double part = 0.0;
-  dispatch_units(L, A, RowSumOp{}, part, red);
+  RowSumOp op;
+  dispatch_units(L, A, op, red);
+  if (L.gid) op.finish(L);
   // singleton state (modularity.cu:459-462), and for a single graph the
   // pass-start communities of the incremental sweep and the row of every
   // entry (the pass loop's flat modularity sweep).  A warp takes 32
@@ -1696,31 +1631,44 @@ __global__ void __launch_bounds__(kThreads)
       }
     }
   }
-  if (!publish_and_check_last(part, 0.0, A, L.sc, red)) return;
-  double msum, unused;
-  sum_partials(A, red, msum, unused);
+  if (!publish_and_check_last(op.m, op.self, op.asq, A, L.sc, red)) return;
+  const double msum = sum_partials(A, 0, red), self = sum_partials(A, 1, red);
+  const double asq = sum_partials(A, 2, red);
   // hubs: finalise their row sums in index order
-  double hs = 0.0;
+  double hs = 0.0, hq = 0.0;
   for (uint32_t i = threadIdx.x; i < A.P.hub_count; i += kThreads) {
     const uint32_t v = A.order[A.P.cls_start[8] + i];
     const float kf = (float)__ldcg(&A.hub_acc[i]);
+    const double kd = (double)kf;
     L.k[v] = kf;
-    L.tot[v] = (double)kf;
-    if (L.tot_alt) L.tot_alt[v] = (double)kf;
+    L.tot[v] = kd;
+    if (L.tot_alt) L.tot_alt[v] = kd;
     A.hub_acc[i] = 0.0;
-    hs += (double)kf;
-    if (L.gid && kf != 0.0f) atomicAdd(&L.gs[L.gid[v]].m_acc, (double)kf);
+    hs += kd;
+    hq += kd * kd;
+    if (L.gid && kf != 0.0f) {
+      atomicAdd(&L.gs[L.gid[v]].m_acc, kd);
+      atomicAdd(&L.gs[L.gid[v]].asq_acc, kd * kd);
+    }
   }
   hs = block_sum(hs, red);
+  hq = block_sum(hq, red);
+  // m and the modularity of the singleton partition: the self-loops are its
+  // intra-community weight, the degrees its totals (its own sweep over the
+  // entries took 1.3 ms of R-MAT 24's 8.5 ms set-up, 545 of 940 us on a batch)
   if (threadIdx.x == 0) {
     const double m64 = (msum + hs) / 2.0;
     const float m = (float)m64;
+    const double sq = asq + hq;
     L.sc->m64 = m64;
     L.sc->m = m;
     L.sc->den = __fmul_rn(__fmul_rn(2.0f, m), m);
+    L.sc->intra = self;
+    L.sc->asq = sq;
+    L.sc->q = (m64 > 0.0) ? (self / (2.0 * m64)) - (sq / (4.0 * m64 * m64)) : 0.0;
     L.sc->done_blocks = 0u;
   }
-  // batched form: every graph's own m (the union's m above is unused)
+  // batched form: every graph's own (the union's above are unused)
   if (L.gid) {
     for (uint32_t g = threadIdx.x; g < L.n_graphs; g += kThreads) {
       GraphState& gs = L.gs[g];
@@ -1729,7 +1677,12 @@ __global__ void __launch_bounds__(kThreads)
       gs.m64 = m64;
       gs.m = m;
       gs.den = __fmul_rn(__fmul_rn(2.0f, m), m);
+      gs.q = (m64 > 0.0) ? (__ldcg(&gs.intra_acc) / (2.0 * m64)) -
+                               (__ldcg(&gs.asq_acc) / (4.0 * m64 * m64))
+                         : 0.0;
       gs.m_acc = 0.0;
+      gs.intra_acc = 0.0;
+      gs.asq_acc = 0.0;
     }
   }
 }
@@ -1789,6 +1742,72 @@ __device__ __forceinline__ double intra_sweep(const LevelView& L, const uint32_t
   return part;
 }
 
+// Batched form: the intra-community weight and the squared totals of every
+// graph still moving.  Their entries are cut into chunks of kUnionChunk
+// (U.start: the graphs' first chunks, an exclusive scan over the active
+// ones); a block takes a consecutive range of chunks, walks the entries flat
+// with their row ids and adds to a graph once per block and graph.  A chunk
+// also carries its share of the graph's totals.  Bound by the entries' bytes
+// and one gather each; the class lists' sweep it replaces spent most of its
+// instructions on per-vertex segmented sums (154 -> 58 us a pass on a batch of
+// 512 graphs).
+__device__ __forceinline__ void union_sweep(const LevelView& L, const uint32_t* rowid,
+                                            const UnionChunks& U, double* red) {
+  const uint64_t total = *U.total;
+  uint32_t c = (uint32_t)(total * blockIdx.x / gridDim.x);
+  const uint32_t c_end = (uint32_t)(total * (blockIdx.x + 1) / gridDim.x);
+  const uint32_t lane = threadIdx.x & 31;
+  while (c < c_end) {  // block-uniform: one graph's chunks of the range
+    uint32_t g = 0, hi = L.n_graphs;  // the last graph starting at or before c
+    for (int round = 0; round < 7 && hi - g > 1; round++) {  // 32^7 > 2^32
+      const uint32_t step = (hi - g + 31) / 32, i = g + lane * step;
+      const unsigned b = __ballot_sync(kFull, lane == 0 || (i < hi && U.start[i] <= c));
+      g += (uint32_t)(__popc(b) - 1) * step;
+      hi = min(hi, g + step);
+    }
+    const uint32_t first = U.start[g];
+    const uint32_t v0 = U.goff[g], v1 = U.goff[g + 1];
+    const uint64_t e0 = L.off[v0], e1 = L.off[v1];
+    const uint32_t chunks = (uint32_t)((e1 - e0 + kUnionChunk - 1) / kUnionChunk);
+    const uint32_t c1 = min(c_end, first + chunks);
+    if (c < first || c1 <= c) {  // the starts are out of step with the rows
+      if (threadIdx.x == 0) atomicExch(&L.sc->error, kErrTableFull);
+      return;
+    }
+    const uint64_t j1 = min(e1, e0 + (uint64_t)(c1 - first) * kUnionChunk);
+    double intra = 0.0, asq = 0.0;
+    for (uint64_t j = e0 + (uint64_t)(c - first) * kUnionChunk + threadIdx.x; j < j1;
+         j += 4 * kThreads) {
+      uint32_t r[4], u[4];
+      float w[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const bool in = j + k * kThreads < j1;
+        r[k] = in ? rowid[j + k * kThreads] : 0u;
+        u[k] = in ? L.col[j + k * kThreads] : 0u;
+        w[k] = in ? L.w[j + k * kThreads] : 0.0f;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (L.comm[r[k]] == L.comm[u[k]]) intra += (double)w[k];
+    }
+    const uint64_t nv = v1 - v0;
+    const uint32_t t1 = v0 + (uint32_t)(nv * (c1 - first) / chunks);
+    for (uint32_t v = v0 + (uint32_t)(nv * (c - first) / chunks) + threadIdx.x; v < t1;
+         v += kThreads) {
+      const double a = L.tot[v];
+      asq += a * a;
+    }
+    intra = block_sum(intra, red);
+    asq = block_sum(asq, red);
+    if (threadIdx.x == 0) {
+      if (intra != 0.0) atomicAdd(&L.gs[g].intra_acc, intra);
+      if (asq != 0.0) atomicAdd(&L.gs[g].asq_acc, asq);
+    }
+    c = c1;
+  }
+}
+
 // Modularity of the current partition (modularity.cu:400-436): the
 // intra-community weight (over the entries with row ids, else over the
 // class lists) and the sum of squared community totals.
@@ -1797,27 +1816,35 @@ __device__ __forceinline__ double intra_sweep(const LevelView& L, const uint32_t
 // moved, and when the previous pass moved fewer than a quarter of the
 // entries it updates the previous intra-community weight from the moved
 // rows only (DeltaIntraOp) instead of sweeping every entry.
+// U (batched form): the active graphs' entry chunks.
 __device__ __forceinline__ void modularity_body(const LevelView& L, const DispatchArgs& A,
                                                 const PassControl& ctl,
                                                 const uint32_t* rowid, uint64_t nnz,
-                                                const uint32_t* cs = nullptr) {
+                                                const uint32_t* cs = nullptr,
+                                                const UnionChunks& U = UnionChunks{}) {
   __shared__ double red[kWarps];
   double part = 0.0;
   // read before this block publishes: the last block rewrites it
   const bool inc = cs && !L.gid && *(volatile uint32_t*)&L.sc->inc_next != 0u;
-  if (inc) {
-    dispatch_units(L, A, DeltaIntraOp{cs}, part, red);
-  } else if (rowid && !L.gid) {
+  if (L.gid) {
+    union_sweep(L, rowid, U, red);
+  } else if (inc) {
+    DeltaIntraOp op{cs};
+    dispatch_units(L, A, op, red);
+    part = op.part;
+  } else if (rowid) {
     part = intra_sweep(L, rowid, nnz, blockIdx.x, gridDim.x);
   } else {
-    dispatch_units(L, A, IntraOp{}, part, red);
+    IntraOp op;
+    dispatch_units(L, A, op, red);
+    part = op.part;
   }
   const uint32_t chunk = (L.n + gridDim.x - 1) / gridDim.x;
   const uint32_t c0 = blockIdx.x * chunk;
   const uint32_t c1 = min(L.n, c0 + chunk);
   double asq = 0.0;
   unsigned long long moved = 0ull;
-  if (!L.gid) {  // the batched form summed a_c^2 with the rows above
+  if (!L.gid) {  // the batched form added them to its graphs above
     for (uint32_t c = c0 + threadIdx.x; c < c1; c += kThreads) {
       const double a = L.tot[c];
       asq += a * a;
@@ -1829,9 +1856,9 @@ __device__ __forceinline__ void modularity_body(const LevelView& L, const Dispat
     for (int o = 16; o > 0; o >>= 1) moved += __shfl_xor_sync(kFull, moved, o);
     if ((threadIdx.x & 31) == 0 && moved) atomicAdd(&L.sc->moved_acc, moved);
   }
-  if (!publish_and_check_last(part, asq, A, L.sc, red)) return;
-  double intra, sq;
-  sum_partials(A, red, intra, sq);
+  if (!publish_and_check_last(part, asq, 0.0, A, L.sc, red)) return;
+  double intra = sum_partials(A, 0, red);
+  const double sq = sum_partials(A, 1, red);
   if (!L.gid) {
     if (threadIdx.x == 0) {
       if (inc) intra += L.sc->intra;  // the pass's change added to the last sweep's sum
@@ -1912,7 +1939,8 @@ __global__ void __launch_bounds__(kThreads, kModPerSM)
   // go into the other copy, which leaves both equal for the next pass
   const LevelView L = step_view(D, io);
   reapply_prev_step(D, io, blockIdx.x, gridDim.x);
-  modularity_body(L, D->A, ctl, D->rowid, D->nnz, D->comm_start);
+  const UnionChunks U{D->chunk_start, D->goff, D->act_cnt ? D->act_cnt + kUnionTotal : nullptr};
+  modularity_body(L, D->A, ctl, D->rowid, D->nnz, D->comm_start, U);
 }
 
 __global__ void pass_control_init_kernel(const PassDesc* __restrict__ D, PassControl ctl) {
@@ -2509,7 +2537,6 @@ DispatchArgs make_args(const uint32_t* order, const DispatchPlan& P,
   A.hub_blk_chunk = hub_map ? hub_map + P.hub_blocks : nullptr;
   A.hub_acc = partials;  // first hub_count doubles; partials follow
   A.partials = partials + P.hub_count;
-  A.act_cnt = nullptr;
   return A;
 }
 
@@ -2849,7 +2876,8 @@ __global__ void class_graph_starts_kernel(const uint32_t* __restrict__ order, Cl
 
 // One block per class: exclusive scan over graphs of the active run
 // lengths -> each active run's place in the compacted list, and the
-// class's active count.  Skipped while the active set is unchanged.
+// class's active count; one more block for the active graphs' entry chunks
+// (the modularity sweep).  Skipped while the active set is unchanged.
 __global__ void __launch_bounds__(1024)
     compact_scan_kernel(const PassDesc* __restrict__ D) {
   const uint32_t* __restrict__ cg = D->cg;
@@ -2861,14 +2889,20 @@ __global__ void __launch_bounds__(1024)
   __shared__ uint32_t warp_tot[32];
   __shared__ uint32_t carry;
   const uint32_t per = G + 1, c = blockIdx.x;
-  const uint32_t* row = cg + c * per;
-  uint32_t* out = cg_new + c * per;
+  const bool chunks = c == kMoveClasses;
+  const uint32_t* row = cg + (chunks ? 0 : c * per);
+  uint32_t* out = chunks ? D->chunk_start : cg_new + c * per;
+  const uint64_t* off = D->L.off;
+  const uint32_t* goff = D->goff;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (threadIdx.x == 0) carry = 0u;
   __syncthreads();
   for (uint32_t b = 0; b < G; b += 1024) {
     const uint32_t g = b + threadIdx.x;
-    const uint32_t len = (g < G && gs[g].active) ? row[g + 1] - row[g] : 0u;
+    uint32_t len = 0u;
+    if (g < G && gs[g].active)
+      len = chunks ? (uint32_t)((off[goff[g + 1]] - off[goff[g]] + kUnionChunk - 1) / kUnionChunk)
+                   : row[g + 1] - row[g];
     uint32_t x = len;  // inclusive warp scan
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -2893,7 +2927,7 @@ __global__ void __launch_bounds__(1024)
     if (threadIdx.x == 1023) carry = before + len;
     __syncthreads();
   }
-  if (threadIdx.x == 0) act_cnt[1 + c] = carry;
+  if (threadIdx.x == 0) act_cnt[chunks ? kUnionTotal : 1 + c] = carry;
 }
 
 // Fills the compacted lists: one thread per output position (blockIdx.y =
@@ -2935,7 +2969,7 @@ cudaError_t launch_class_graph_starts(const uint32_t* order, const DispatchPlan&
 }
 
 cudaError_t launch_compact_active(const PassDesc* D, cudaStream_t st) {
-  (count_launches(1), compact_scan_kernel<<<kMoveClasses, 1024, 0, st>>>(D));
+  (count_launches(1), compact_scan_kernel<<<kMoveClasses + 1, 1024, 0, st>>>(D));
   const dim3 grid(sm_count() * 2, kMoveClasses);
   (count_launches(1), compact_copy_kernel<<<grid, 256, 0, st>>>(D));
   return cudaGetLastError();

@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     S.D.L.sc = &S.sc;
     S.G = A.L;
     S.G.sc = &S.sc;
-    S.D.A.act_cnt = S.D.act_cnt = S.cls_own;
+    S.D.act_cnt = S.cls_own;
     S.D.A.order = M.order;
     S.D.prop = M.prop;
     S.D.comm_start = nullptr;
