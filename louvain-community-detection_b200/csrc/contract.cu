@@ -43,7 +43,10 @@ constexpr int kWarpSlots = 256;                 // class W table
 constexpr int kMidSlots = 2048;                 // class B table
 constexpr int kMidSmem = kMidSlots * 12 + kThreads * 16;
 constexpr int kBlockSlots = 8192;               // class B2 table
-constexpr int kBlockSmem = kBlockSlots * 12 + kThreads * 16;
+// Class B2's tables leave room for two blocks per SM whatever their threads:
+// at 256 an SM ran 16 warps on chains of 16 entries a thread.
+constexpr int kB2Threads = 512;
+constexpr int kBlockSmem = kBlockSlots * 12 + kB2Threads * 16;
 static_assert(kMergeMidMax * 3 / 2 + 1 <= kMidSlots &&
                   kMergeBlockMax * 3 / 2 + 1 <= kBlockSlots,
               "tables keep load factor <= 2/3");
@@ -355,6 +358,7 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+template <int NT = kThreads>
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t* sm,
                                                     uint32_t* total) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -368,22 +372,23 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t* sm,
   __syncthreads();
   if (threadIdx.x == 0) {
     uint32_t run = 0;
-    for (int i = 0; i < kWarps; i++) {
+    for (int i = 0; i < NT / 32; i++) {
       uint32_t t = sm[i];
       sm[i] = run;
       run += t;
     }
-    sm[kWarps] = run;
+    sm[NT / 32] = run;
   }
   __syncthreads();
   const uint32_t r = sm[wib] + incl - x;
-  *total = sm[kWarps];
+  *total = sm[NT / 32];
   __syncthreads();
   return r;
 }
 
 // Inserts positions [lo, hi) of a community's flattened edge range into a
-// table; members are staged through shared memory 256 at a time.
+// table; members are staged through shared memory NT at a time.
+template <int NT = kThreads>
 __device__ __forceinline__ void insert_range(const Ctx& C, uint32_t m0,
                                              uint32_t msz, uint64_t seg,
                                              uint64_t total, uint64_t lo,
@@ -415,21 +420,21 @@ __device__ __forceinline__ void insert_range(const Ctx& C, uint32_t m0,
       s_off[threadIdx.x] = 0;
     }
     __syncthreads();
-    const uint32_t nvalid = min((uint32_t)kThreads, msz - k0);
+    const uint32_t nvalid = min((uint32_t)NT, msz - k0);
     const uint64_t chunk_end =
-        (k0 + kThreads < msz) ? min(hi, C.mstart[m0 + k0 + kThreads] - seg) : hi;
+        (k0 + NT < msz) ? min(hi, C.mstart[m0 + k0 + NT] - seg) : hi;
     // kWaves waves of the block at a time, every load of a batch issued
     // before its first insert
     constexpr int kWaves = 4;
-    for (uint64_t p0 = pos; p0 < chunk_end; p0 += (uint64_t)kWaves * kThreads) {
+    for (uint64_t p0 = pos; p0 < chunk_end; p0 += (uint64_t)kWaves * NT) {
       uint32_t key[kWaves];
       float wt[kWaves];
 #pragma unroll
       for (int k = 0; k < kWaves; k++) {
-        const uint64_t p = p0 + (uint64_t)k * kThreads + threadIdx.x;
+        const uint64_t p = p0 + (uint64_t)k * NT + threadIdx.x;
         key[k] = kEmptyKey;
         wt[k] = 0.0f;
-        if (p0 + (uint64_t)k * kThreads >= chunk_end) continue;  // block-uniform
+        if (p0 + (uint64_t)k * NT >= chunk_end) continue;  // block-uniform
         if (p < chunk_end) {
           int a = 0, b = (int)nvalid - 1;
           while (a < b) {
@@ -456,7 +461,7 @@ __device__ __forceinline__ void insert_range(const Ctx& C, uint32_t m0,
       }
     }
     pos = chunk_end;
-    k0 += kThreads;
+    k0 += NT;
     __syncthreads();
   }
   (void)total;
@@ -464,31 +469,31 @@ __device__ __forceinline__ void insert_range(const Ctx& C, uint32_t m0,
 
 // Classes B (SLOTS = 2048: <= 1024 entries) and B2 (8192: <= 4096): one
 // block per community, shared table of up to SLOTS slots.
-template <int SLOTS>
-__global__ void __launch_bounds__(kThreads)
+template <int SLOTS, int NT>
+__global__ void __launch_bounds__(NT)
     merge_block_kernel(Ctx C, const uint32_t* list, uint32_t count) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* vals = reinterpret_cast<double*>(smem_raw);
   uint64_t* s_start = reinterpret_cast<uint64_t*>(smem_raw + SLOTS * 8);
-  uint64_t* s_off = s_start + kThreads;
-  uint32_t* keys = reinterpret_cast<uint32_t*>(smem_raw + SLOTS * 8 + kThreads * 16);
-  __shared__ uint32_t scan_sm[kWarps + 1];
+  uint64_t* s_off = s_start + NT;
+  uint32_t* keys = reinterpret_cast<uint32_t*>(smem_raw + SLOTS * 8 + NT * 16);
+  __shared__ uint32_t scan_sm[NT / 32 + 1];
   for (uint32_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
     const uint32_t cn = list[idx];
     const uint32_t c = C.comm_list[cn];
     const uint32_t m0 = C.mem_off[c], msz = C.comm_sz[c];
     const uint64_t seg = C.mstart[m0];
     const uint64_t total = C.mstart[m0 + msz] - seg;
-    // class B rows hold > 128 entries, so tv >= 256 = kThreads
-    const uint32_t tv = table_size_for((uint32_t)total, SLOTS);
-    for (uint32_t i = threadIdx.x; i < tv; i += kThreads) {
+    // at least a slot per thread
+    const uint32_t tv = max(table_size_for((uint32_t)total, SLOTS), (uint32_t)NT);
+    for (uint32_t i = threadIdx.x; i < tv; i += NT) {
       keys[i] = kEmptyKey;
       vals[i] = 0.0;
     }
     __syncthreads();
     double hot_acc = 0.0;
     bool hot_seen = false;
-    insert_range(C, m0, msz, seg, total, 0, total, keys, vals, tv - 1, s_start, s_off, cn,
+    insert_range<NT>(C, m0, msz, seg, total, 0, total, keys, vals, tv - 1, s_start, s_off, cn,
                  hot_acc, hot_seen);
     // every warp adds its share of the new self-loop (FP64 sums of FP32
     // weights are exact in any order): no block-wide sum first
@@ -497,11 +502,11 @@ __global__ void __launch_bounds__(kThreads)
       atomicAdd(&vals[table_insert(keys, tv - 1, cn, C.err)], hot_acc);
     __syncthreads();
     // emit: thread t owns slots [t*per, t*per + per)
-    const uint32_t per = tv / kThreads;
+    const uint32_t per = tv / NT;
     uint32_t local = 0;
     for (uint32_t i = 0; i < per; i++) local += keys[threadIdx.x * per + i] != kEmptyKey;
     uint32_t tot;
-    uint32_t pos = block_excl_scan(local, scan_sm, &tot);
+    uint32_t pos = block_excl_scan<NT>(local, scan_sm, &tot);
     for (uint32_t i = 0; i < per; i++) {
       const uint32_t sl = threadIdx.x * per + i;
       const uint32_t key = keys[sl];
@@ -797,11 +802,11 @@ unsigned gridcap(uint64_t work, unsigned per_sm) {
 }  // namespace
 
 cudaError_t configure_contract_kernels() {
-  cudaError_t e = cudaFuncSetAttribute(merge_block_kernel<kMidSlots>,
+  cudaError_t e = cudaFuncSetAttribute(merge_block_kernel<kMidSlots, kThreads>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kMidSmem);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(merge_block_kernel<kBlockSlots>,
+  return cudaFuncSetAttribute(merge_block_kernel<kBlockSlots, kB2Threads>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, kBlockSmem);
 }
 
@@ -910,12 +915,12 @@ cudaError_t contract_back(const LevelView& L, uint64_t nnz, ContractBuffers& B,
     LV_TRY(cudaGetLastError());
   }
   if (cntM) {
-    (count_launches(1), merge_block_kernel<kMidSlots><<<gridcap(cntM, 7), kThreads, kMidSmem, st>>>(
+    (count_launches(1), merge_block_kernel<kMidSlots, kThreads><<<gridcap(cntM, 7), kThreads, kMidSmem, st>>>(
         C, B.comm_cls + cntW, cntM));
     LV_TRY(cudaGetLastError());
   }
   if (cntB2) {
-    (count_launches(1), merge_block_kernel<kBlockSlots><<<gridcap(cntB2, 2), kThreads, kBlockSmem, st>>>(
+    (count_launches(1), merge_block_kernel<kBlockSlots, kB2Threads><<<gridcap(cntB2, 2), kB2Threads, kBlockSmem, st>>>(
         C, B.comm_cls + cntW + cntM, cntB2));
     LV_TRY(cudaGetLastError());
   }

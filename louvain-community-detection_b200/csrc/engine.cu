@@ -2124,8 +2124,9 @@ constexpr uint64_t kSmallLaterEntries = 32768;
 constexpr uint64_t kSmallOneEntries = 1536;
 constexpr uint32_t kSmallOneVertices = 64;
 // A refused launch costs a host wait, 30 us: a contracted level whose entries
-// are not known yet is offered only when the level before had at most this
-// many (contractions of late levels shrink the entries four- to tenfold).
+// are not known yet is offered only when it cannot have too many (a row has
+// at most one entry per vertex) or the level before had at most this many
+// (contractions of late levels shrink the entries four- to tenfold).
 constexpr uint64_t kSmallPrevEntries = 1ull << 18;
 
 static uint64_t small_max_entries(const lv_engine* E) {
@@ -2138,7 +2139,9 @@ static uint64_t small_max_entries(const lv_engine* E) {
 static bool small_eligible(const lv_engine* E) {
   return E->cfg.use_graphs && !E->profiling && !E->batch && !use_level_kernel(E) &&
          !E->cfg.contract_sort && !E->cfg.apply_launch && !E->level_ready && !E->small_off &&
-         E->n > 0 && E->n <= kSmallMaxN && E->e <= (E->agg_pending ? kSmallPrevEntries : small_max_entries(E));
+         E->n > 0 && E->n <= kSmallMaxN &&
+         (E->agg_pending ? E->e <= kSmallPrevEntries || (uint64_t)E->n * E->n <= small_max_entries(E)
+                         : E->e <= small_max_entries(E));
 }
 
 // Runs the engine's level (with move_only its passes, else every level to the

@@ -1535,34 +1535,58 @@ __device__ __forceinline__ void unit_hub(const LevelView& L, const DispatchArgs&
   if (threadIdx.x == 0) op.hub(L, A, hi, x);
 }
 
-// Deterministic block reduction into partials, then the last block to
-// finish sums all partials in index order.
+// Deterministic block reduction of three sums into partials, then the last
+// of the nblk blocks to finish sums all partials in index order.
 __device__ __forceinline__ bool publish_and_check_last(double a, double b, double c,
-                                                       const DispatchArgs& A,
-                                                       LevelScalars* sc,
-                                                       double* red) {
+                                                       const DispatchArgs& A, LevelScalars* sc,
+                                                       uint32_t nblk) {
+  __shared__ double part[kWarps][3];
   __shared__ bool last;
-  double ra = block_sum(a, red);
-  double rb = block_sum(b, red);
-  double rc = block_sum(c, red);
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  a = group_sum<32>(a);
+  b = group_sum<32>(b);
+  c = group_sum<32>(c);
+  if (lane == 0) {
+    part[wib][0] = a;
+    part[wib][1] = b;
+    part[wib][2] = c;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    A.partials[blockIdx.x] = ra;
-    A.partials[gridDim.x + blockIdx.x] = rb;
-    A.partials[2 * gridDim.x + blockIdx.x] = rc;
+    double s[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int w = 0; w < kWarps; w++)
+#pragma unroll
+      for (int i = 0; i < 3; i++) s[i] += part[w][i];
+    double* p = A.partials + 3ull * blockIdx.x;
+    p[0] = s[0];
+    p[1] = s[1];
+    p[2] = s[2];
     __threadfence();
     const uint32_t t = atomicAdd(&sc->done_blocks, 1u);
-    last = (t == gridDim.x - 1);
+    last = (t == nblk - 1);
   }
   __syncthreads();
   if (last) __threadfence();
   return last;
 }
 
-__device__ __forceinline__ double sum_partials(const DispatchArgs& A, int which, double* red) {
-  double x = 0.0;
-  for (uint32_t i = threadIdx.x; i < gridDim.x; i += kThreads)
-    x += __ldcg(&A.partials[which * gridDim.x + i]);
-  return block_sum(x, red);
+struct Sums3 {
+  double a, b, c;
+};
+// The partials' sums, valid in thread 0.
+__device__ __forceinline__ Sums3 sum_partials(const DispatchArgs& A, uint32_t nblk, double* red) {
+  Sums3 s{0.0, 0.0, 0.0};
+  for (uint32_t i = threadIdx.x; i < nblk; i += kThreads) {
+    const double* p = A.partials + 3ull * i;
+    s.a += __ldcg(p);
+    s.b += __ldcg(p + 1);
+    s.c += __ldcg(p + 2);
+  }
+  s.a = block_sum(s.a, red);
+  s.b = block_sum(s.b, red);
+  s.c = block_sum(s.c, red);
+  return s;
 }
 
 // Units of the class lists: every class's units are split into one
@@ -1631,9 +1655,8 @@ __global__ void __launch_bounds__(kThreads)
       }
     }
   }
-  if (!publish_and_check_last(op.m, op.self, op.asq, A, L.sc, red)) return;
-  const double msum = sum_partials(A, 0, red), self = sum_partials(A, 1, red);
-  const double asq = sum_partials(A, 2, red);
+  if (!publish_and_check_last(op.m, op.self, op.asq, A, L.sc, gridDim.x)) return;
+  const Sums3 all = sum_partials(A, gridDim.x, red);
   // hubs: finalise their row sums in index order
   double hs = 0.0, hq = 0.0;
   for (uint32_t i = threadIdx.x; i < A.P.hub_count; i += kThreads) {
@@ -1657,15 +1680,15 @@ __global__ void __launch_bounds__(kThreads)
   // intra-community weight, the degrees its totals (its own sweep over the
   // entries took 1.3 ms of R-MAT 24's 8.5 ms set-up, 545 of 940 us on a batch)
   if (threadIdx.x == 0) {
-    const double m64 = (msum + hs) / 2.0;
+    const double m64 = (all.a + hs) / 2.0;
     const float m = (float)m64;
-    const double sq = asq + hq;
+    const double sq = all.c + hq;
     L.sc->m64 = m64;
     L.sc->m = m;
     L.sc->den = __fmul_rn(__fmul_rn(2.0f, m), m);
-    L.sc->intra = self;
+    L.sc->intra = all.b;
     L.sc->asq = sq;
-    L.sc->q = (m64 > 0.0) ? (self / (2.0 * m64)) - (sq / (4.0 * m64 * m64)) : 0.0;
+    L.sc->q = (m64 > 0.0) ? (all.b / (2.0 * m64)) - (sq / (4.0 * m64 * m64)) : 0.0;
     L.sc->done_blocks = 0u;
   }
   // batched form: every graph's own (the union's above are unused)
@@ -1752,10 +1775,10 @@ __device__ __forceinline__ double intra_sweep(const LevelView& L, const uint32_t
 // instructions on per-vertex segmented sums (154 -> 58 us a pass on a batch of
 // 512 graphs).
 __device__ __forceinline__ void union_sweep(const LevelView& L, const uint32_t* rowid,
-                                            const UnionChunks& U, double* red) {
+                                            const UnionChunks& U, uint32_t nblk, double* red) {
   const uint64_t total = *U.total;
-  uint32_t c = (uint32_t)(total * blockIdx.x / gridDim.x);
-  const uint32_t c_end = (uint32_t)(total * (blockIdx.x + 1) / gridDim.x);
+  uint32_t c = (uint32_t)(total * blockIdx.x / nblk);
+  const uint32_t c_end = (uint32_t)(total * (blockIdx.x + 1) / nblk);
   const uint32_t lane = threadIdx.x & 31;
   while (c < c_end) {  // block-uniform: one graph's chunks of the range
     uint32_t g = 0, hi = L.n_graphs;  // the last graph starting at or before c
@@ -1820,26 +1843,26 @@ __device__ __forceinline__ void union_sweep(const LevelView& L, const uint32_t* 
 __device__ __forceinline__ void modularity_body(const LevelView& L, const DispatchArgs& A,
                                                 const PassControl& ctl,
                                                 const uint32_t* rowid, uint64_t nnz,
-                                                const uint32_t* cs = nullptr,
+                                                uint32_t nblk, const uint32_t* cs = nullptr,
                                                 const UnionChunks& U = UnionChunks{}) {
   __shared__ double red[kWarps];
   double part = 0.0;
   // read before this block publishes: the last block rewrites it
   const bool inc = cs && !L.gid && *(volatile uint32_t*)&L.sc->inc_next != 0u;
   if (L.gid) {
-    union_sweep(L, rowid, U, red);
+    union_sweep(L, rowid, U, nblk, red);
   } else if (inc) {
     DeltaIntraOp op{cs};
     dispatch_units(L, A, op, red);
     part = op.part;
   } else if (rowid) {
-    part = intra_sweep(L, rowid, nnz, blockIdx.x, gridDim.x);
+    part = intra_sweep(L, rowid, nnz, blockIdx.x, nblk);
   } else {
     IntraOp op;
     dispatch_units(L, A, op, red);
     part = op.part;
   }
-  const uint32_t chunk = (L.n + gridDim.x - 1) / gridDim.x;
+  const uint32_t chunk = (L.n + nblk - 1) / nblk;
   const uint32_t c0 = blockIdx.x * chunk;
   const uint32_t c1 = min(L.n, c0 + chunk);
   double asq = 0.0;
@@ -1856,10 +1879,11 @@ __device__ __forceinline__ void modularity_body(const LevelView& L, const Dispat
     for (int o = 16; o > 0; o >>= 1) moved += __shfl_xor_sync(kFull, moved, o);
     if ((threadIdx.x & 31) == 0 && moved) atomicAdd(&L.sc->moved_acc, moved);
   }
-  if (!publish_and_check_last(part, asq, 0.0, A, L.sc, red)) return;
-  double intra = sum_partials(A, 0, red);
-  const double sq = sum_partials(A, 1, red);
+  if (!publish_and_check_last(part, asq, 0.0, A, L.sc, nblk)) return;
   if (!L.gid) {
+    const Sums3 all = sum_partials(A, nblk, red);
+    double intra = all.a;
+    const double sq = all.b;
     if (threadIdx.x == 0) {
       if (inc) intra += L.sc->intra;  // the pass's change added to the last sweep's sum
       const unsigned long long mv = cs ? atomicExch(&L.sc->moved_acc, 0ull) : 0ull;
@@ -1926,7 +1950,7 @@ __device__ __forceinline__ void modularity_body(const LevelView& L, const Dispat
 
 __global__ void __launch_bounds__(kThreads)
     modularity_kernel(LevelView L, DispatchArgs A, PassControl ctl) {
-  modularity_body(L, A, ctl, nullptr, 0);
+  modularity_body(L, A, ctl, nullptr, 0, gridDim.x);
 }
 
 // The modularity sweep of a pass (level and stop-rule limits from the
@@ -1938,9 +1962,19 @@ __global__ void __launch_bounds__(kThreads, kModPerSM)
   // reads the copy holding every move of the pass; the last step's moves
   // go into the other copy, which leaves both equal for the next pass
   const LevelView L = step_view(D, io);
-  reapply_prev_step(D, io, blockIdx.x, gridDim.x);
+  // small levels are swept by fewer blocks, 2,048 entries or vertices each (a
+  // union chunk): 888 arrivals on one counter took 4 of 8.8 us
+  uint32_t nblk = gridDim.x;
+  if (L.gid) {
+    nblk = min(nblk, max(D->act_cnt[kUnionTotal], 1u));
+  } else if (!D->comm_start) {
+    const uint64_t work = (max(D->nnz, (uint64_t)L.n) + 2047) / 2048;
+    nblk = (uint32_t)min((uint64_t)nblk, max(work, (uint64_t)1));
+  }
+  if (blockIdx.x >= nblk) return;
+  reapply_prev_step(D, io, blockIdx.x, nblk);
   const UnionChunks U{D->chunk_start, D->goff, D->act_cnt ? D->act_cnt + kUnionTotal : nullptr};
-  modularity_body(L, D->A, ctl, D->rowid, D->nnz, D->comm_start, U);
+  modularity_body(L, D->A, ctl, D->rowid, D->nnz, nblk, D->comm_start, U);
 }
 
 __global__ void pass_control_init_kernel(const PassDesc* __restrict__ D, PassControl ctl) {
