@@ -2371,15 +2371,17 @@ __global__ void bucket_ids_kernel(const uint64_t* off, uint32_t n, uint8_t* out)
 // FP64 modularity of an arbitrary partition: one sweep over the entries
 // (community totals, intra-community weight, total weight), then the squared
 // totals.  Bound by the entries' columns and weights from memory and one
-// 4-byte gather of the neighbour's community each.  A warp takes 32
-// consecutive rows as one flat range of entries, so every load but the
-// gather is coalesced (a thread per row read a sector per entry, and each
-// row twice: 530 -> 207 us for 1 M vertices and 14 M entries).  Rows above
-// kPartLong entries go to a list of (row, chunk) pairs that the whole grid
-// shares afterwards.  acc: [0] intra, [1] squared totals, [2] all weight,
+// 4-byte gather of the neighbour's community each.  Eight lanes take a row,
+// four rows a warp at a time (a thread per row read a sector per entry, and
+// each row twice: 530 us for 1 M vertices and 14 M entries; a warp's 32 rows as
+// one flat range with segmented sums 207 us; eight lanes 192 us, and with the
+// large communities' totals gathered per block first 91 us).  Rows above kPartLong
+// entries go to a list of (row, chunk) pairs that the whole grid shares
+// afterwards.  acc: [0] intra, [1] squared totals, [2] all weight,
 // [3] vertices with a community id >= n (skipped: the caller refuses the
 // partition).
-constexpr uint32_t kPartLong = 1024;
+constexpr int kPartCache = 1024;
+constexpr uint32_t kPartLong = 256;
 constexpr uint32_t kPartChunk = 4096;
 struct PartArgs {
   const uint32_t* part;
@@ -2414,7 +2416,15 @@ __device__ __forceinline__ void part_range(const LevelView& L, const PartArgs& P
 __global__ void __launch_bounds__(kThreads)
     part_sweep_kernel(const LevelView L, PartArgs P) {
   __shared__ double red[kWarps];
-  __shared__ double rsum[kWarps][32];
+  // totals of the communities the block met first, added to memory once: a
+  // large community's rows would queue on one address
+  __shared__ uint32_t ckey[kPartCache];
+  __shared__ double csum[kPartCache];
+  for (int i = threadIdx.x; i < kPartCache; i += kThreads) {
+    ckey[i] = kEmptyKey;
+    csum[i] = 0.0;
+  }
+  __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   double intra = 0.0, all = 0.0, bad = 0.0;
   const uint64_t step = (uint64_t)gridDim.x * kThreads;
@@ -2454,63 +2464,40 @@ __global__ void __launch_bounds__(kThreads)
       row = group_sum<32>(row);
       if (lane == 0 && row != 0.0) atomicAdd(&P.tot[rp], row);
     }
-    uint32_t incl = len;
+    const int gl = lane & 7;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(kFull, incl, o);
-      if (lane >= o) incl += y;
-    }
-    const uint32_t pre = incl - len, total = __shfl_sync(kFull, incl, 31);
-    rsum[wib][lane] = 0.0;
-    __syncwarp();
-    constexpr int kWaves = 4;
-    for (uint32_t f0 = 0; f0 < total; f0 += 32 * kWaves) {
-      uint32_t q[kWaves], c[kWaves], pq[kWaves];
-      float w[kWaves];
+    for (int q = 0; q < 8; q++) {  // rows v0 + 4 q .. + 3
+      const int r = q * 4 + (lane >> 3);
+      const uint64_t rs = __shfl_sync(kFull, s, r);
+      const uint32_t rl = __shfl_sync(kFull, len, r), rp = __shfl_sync(kFull, p, r);
+      double row = 0.0;
+      for (uint32_t j0 = gl; j0 < rl; j0 += 32) {
+        uint32_t c[4];
+        float w[4];
 #pragma unroll
-      for (int k = 0; k < kWaves; k++) {
-        const uint32_t f = f0 + k * 32 + lane;
-        uint32_t lo = 0, hi = 31;  // the last row starting at or before f
-#pragma unroll
-        for (int it = 0; it < 5; it++) {
-          const uint32_t mid = (lo + hi + 1) >> 1;
-          if (__shfl_sync(kFull, pre, mid) <= f) lo = mid; else hi = mid - 1;
-          if (hi < lo) hi = lo;
+        for (int k = 0; k < 4; k++) {
+          const uint32_t j = j0 + k * 8;
+          c[k] = j < rl ? L.col[rs + j] : 0u;
+          w[k] = j < rl ? L.w[rs + j] : 0.0f;
         }
-        const uint64_t rs = __shfl_sync(kFull, s, lo);
-        const uint32_t rpre = __shfl_sync(kFull, pre, lo);
-        pq[k] = __shfl_sync(kFull, p, lo);
-        q[k] = f < total ? lo : 32u;
-        c[k] = 0u;
-        w[k] = 0.0f;
-        if (f < total) {
-          c[k] = L.col[rs + (f - rpre)];
-          w[k] = L.w[rs + (f - rpre)];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          row += (double)w[k];
+          if (P.part[c[k]] == rp) intra += (double)w[k];
         }
       }
-#pragma unroll
-      for (int k = 0; k < kWaves; k++)
-        if (q[k] < 32u && P.part[c[k]] == pq[k]) intra += (double)w[k];
-#pragma unroll
-      for (int k = 0; k < kWaves; k++) {
-        if (f0 + k * 32 >= total) break;  // warp-uniform
-        double x = (double)w[k];
-        all += x;
-        // segmented suffix sum: the first lane of a row's run gets the run
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const double y = __shfl_down_sync(kFull, x, o);
-          const uint32_t yq = __shfl_down_sync(kFull, q[k], o);
-          if (lane + o < 32 && yq == q[k]) x += y;
-        }
-        const uint32_t before = __shfl_up_sync(kFull, q[k], 1);
-        if (q[k] < 32u && (lane == 0 || before != q[k])) rsum[wib][q[k]] += x;
-        __syncwarp();
+      all += row;
+      row = group_sum<8>(row);
+      if (gl == 0 && row != 0.0) {
+        const uint32_t h = hash_slot(rp, kPartCache - 1);
+        const uint32_t was = atomicCAS(&ckey[h], kEmptyKey, rp);
+        atomicAdd(was == kEmptyKey || was == rp ? &csum[h] : &P.tot[rp], row);
       }
     }
-    if (len && rsum[wib][lane] != 0.0) atomicAdd(&P.tot[p], rsum[wib][lane]);
-    __syncwarp();
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kPartCache; i += kThreads)
+    if (ckey[i] != kEmptyKey && csum[i] != 0.0) atomicAdd(&P.tot[ckey[i]], csum[i]);
   intra = block_sum(intra, red);
   all = block_sum(all, red);
   bad = block_sum(bad, red);

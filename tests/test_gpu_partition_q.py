@@ -1,6 +1,8 @@
 """Modularity of a given partition (lv_modularity_fp64) over rows of every
-length its sweep treats apart: empty, short, above 1,024 entries (listed in
-chunks of 4,096 that all blocks share) and more chunks than the list holds.
+length its sweep treats apart: empty, short, above 256 entries (listed in
+chunks of 4,096 that all blocks share) and more chunks than the list holds;
+partitions of one community, of many and of more than a block's cache of
+1,024 totals holds.
 Reference: the same sums in numpy, FP64.  The FP32 weights' FP64 sums are
 exact; only the squared totals round (n terms, each to 2^-53 of a sum that is
 at most 1 after the division), so 1e-12 is far above the difference."""
@@ -30,7 +32,7 @@ def _q(n, off, col, w, part):
 
 
 @pytest.mark.parametrize("degrees", [
-    [3], [0, 0, 5, 0], [1] * 31, [2] * 33, [1024] * 4, [1025, 1, 0, 4096, 4097, 9000] * 7,
+    [3], [0, 0, 5, 0], [1] * 31, [2] * 33, [255, 256, 257, 8], [1024] * 4, [6] * 9000, [1025, 1, 0, 4096, 4097, 9000] * 7,
     [60_000, 50_000, 7], [0] * 300 + [13] * 700 + [2000]])
 def test_q_of_partition_equals_numpy(degrees):
     n, off, col, w = _csr(degrees, seed=len(degrees))
