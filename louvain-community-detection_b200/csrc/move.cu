@@ -675,34 +675,28 @@ __device__ __forceinline__ void load_row_vec(const LevelView& L, uint64_t s, uin
   }
 }
 
-// The candidates of the keys a thread claimed while its entries went into
-// a complete table: entry slot i's table slot is the i-th 16-bit field of
-// `slots` (bit i of `owned` set); the key is read back from the table, so
-// the entries' registers are free once they are inserted.  Four at a time,
-// so their gathers overlap; each slot is emptied after it is read, which
-// leaves the table clean without a scan of its empty slots.
-template <int NE>
-__device__ __forceinline__ void claim_slot(uint32_t (&slots)[(NE + 1) / 2], uint32_t& owned,
-                                           int i, uint32_t slot) {
-  owned |= 1u << i;
+// The candidates of the keys a warp claimed while its entries went into a
+// complete table (exactly one warp claims a key): their slots sit in the
+// warp's list, so the lanes share them evenly, two at a time, and each slot
+// is emptied after it is read, which leaves the table clean without a scan of
+// its empty slots.  (With a thread evaluating its own claims, a warp walked
+// all its insert rounds for the one or two candidates a lane has once
+// communities have formed: 5.5-7 of 21 thousand cycles a vertex.)
+template <int PREC>
+__device__ __forceinline__ typename BestOf<PREC>::T eval_claims(const LevelView& L,
+                                                                const GainCtx& g, uint32_t* keys,
+                                                                double* vals,
+                                                                const uint16_t* list,
+                                                                uint32_t cnt) {
+  typename BestOf<PREC>::T best{};
+#pragma unroll 1
+  for (uint32_t i0 = threadIdx.x & 31; i0 < cnt; i0 += 64) {
+    uint32_t szc[2], slot[2], c[2];
+    double ec[2], ac[2];
 #pragma unroll
-  for (int j = 0; j < (NE + 1) / 2; j++)  // i is a constant of the unrolled caller
-    if (j == (i >> 1)) slots[j] |= slot << (16 * (i & 1));
-}
-template <int PREC, int NE>
-__device__ __forceinline__ typename BestOf<PREC>::T eval_owned(
-    const LevelView& L, const GainCtx& g, uint32_t* keys, double* vals,
-    const uint32_t (&slots)[(NE + 1) / 2], uint32_t owned, typename BestOf<PREC>::T best) {
-#pragma unroll
-  for (int i0 = 0; i0 < NE; i0 += 4) {
-    if (((owned >> i0) & 0xFu) == 0u) continue;
-    uint32_t szc[4], slot[4], c[4];
-    double ec[4], ac[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int i = i0 + q;
-      if (i < NE && (owned >> i & 1u)) {
-        slot[q] = (slots[i >> 1] >> (16 * (i & 1))) & 0xFFFFu;
+    for (int q = 0; q < 2; q++) {
+      if (i0 + 32 * q < cnt) {
+        slot[q] = list[i0 + 32 * q];
         c[q] = keys[slot[q]];
         ec[q] = vals[slot[q]];
         szc[q] = candidate_size(L, g, c[q]);
@@ -710,27 +704,14 @@ __device__ __forceinline__ typename BestOf<PREC>::T eval_owned(
       }
     }
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int i = i0 + q;
-      if (i < NE && (owned >> i & 1u)) {
+    for (int q = 0; q < 2; q++) {
+      if (i0 + 32 * q < cnt) {
         best = best_max(best, candidate_loaded<PREC>(g, c[q], ec[q], szc[q], ac[q]));
         keys[slot[q]] = kEmptyKey;
         vals[slot[q]] = 0.0;
       }
     }
   }
-  return best;
-}
-
-// The own community's candidate, for the thread that claimed its slot.
-template <int PREC>
-__device__ __forceinline__ typename BestOf<PREC>::T eval_own_slot(
-    const LevelView& L, const GainCtx& g, uint32_t* keys, double* vals, uint32_t slot,
-    typename BestOf<PREC>::T best) {
-  const double ec = vals[slot];
-  best = best_max(best, candidate_loaded<PREC>(g, g.cv, ec, g.szv, L.tot[g.cv]));
-  keys[slot] = kEmptyKey;
-  vals[slot] = 0.0;
   return best;
 }
 
@@ -881,8 +862,8 @@ __device__ __forceinline__ double block_sum(double x, double* red) {
 
 // Loads entries [lo, end) of row s (at most MAXW waves of the block) into
 // registers -- every load issued before any is used -- then inserts them
-// into a table (clear it before, synchronise after).  cu / wt / owned come
-// back as eval_owned reads them.
+// into a table (clear it before, synchronise after).  The slots of the keys
+// this warp put in go to its list (eval_claims), `cnt` of them.
 template <int MAXW, int RULE, int NT>
 __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t s,
                                                    uint64_t lo, uint64_t end,
@@ -890,12 +871,11 @@ __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t 
                                                    uint32_t* keys, double* vals,
                                                    uint32_t mask, double& own,
                                                    double& hot, bool& hot_seen,
-                                                   uint32_t (&slots)[(MAXW + 1) / 2],
-                                                   uint32_t& owned) {
+                                                   uint16_t* list, uint32_t& cnt) {
   uint32_t cu[MAXW];
   float wt[MAXW];
   unsigned self_mask = 0u;
-  owned = 0u;
+  const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
 #pragma unroll
   for (int k = 0; k < MAXW; k++) {
     const uint64_t j = lo + (uint64_t)k * NT + threadIdx.x;
@@ -924,27 +904,36 @@ __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t 
       hot_seen = true;
       if (RULE == LV_RULE_CUDA_I && !(self_mask >> k & 1u)) own += (double)wt[k];
     }
+    bool claimed = false;
+    uint32_t slot = 0;
     if (ins) {
-      bool claimed;
-      const uint32_t slot = table_claim(keys, mask, cu[k], L.sc, claimed);
+      slot = table_claim(keys, mask, cu[k], L.sc, claimed);
       atomicAdd(&vals[slot], (double)wt[k]);
-      if (claimed) claim_slot<MAXW>(slots, owned, k, slot);
     }
+    const unsigned cb = __ballot_sync(kFull, claimed);
+    if (claimed) list[cnt + __popc(cb & lt)] = (uint16_t)slot;
+    cnt += __popc(cb);
   }
 }
+
+// Claims a warp of a block of nt threads can make on a row of maxdeg entries
+// (and the own community's).
+__host__ __device__ constexpr int claim_list(int maxdeg, int nt) { return (maxdeg + nt - 1) / nt * 32 + 2; }
 
 // A block of NT threads per vertex of at most MAXDEG entries, T-slot table.
 template <int MODE, int NT = kThreads, int T = kHubSmemSlots, int MAXDEG = (int)kHubSmemMaxDeg>
 __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int cls, uint32_t bid,
                                            uint32_t nblk, unsigned char* smem_raw,
                                            typename BestOf<ModeOf<MODE>::kPrec>::T* red_best,
-                                           double* red_own, const StepIO io = StepIO{}) {
+                                           double* red_own, uint16_t* claims,
+                                           const StepIO io = StepIO{}) {
   constexpr int RULE = ModeOf<MODE>::kRule, PREC = ModeOf<MODE>::kPrec;
   using K = typename BestOf<PREC>::T;
   const LevelView L = step_view(D, io);
   const uint32_t s0 = D->A.P.cls_start[cls];
   const uint32_t* __restrict__ verts = D->A.order + s0;
   uint32_t* __restrict__ prop = D->prop + s0;
+  uint16_t* list = claims + (threadIdx.x >> 5) * claim_list(MAXDEG, NT);
   const uint32_t count = D->act_cnt ? D->act_cnt[cls] : D->A.P.cls_start[cls + 1] - s0;
   constexpr int MAXW = (MAXDEG + NT - 1) / NT;
   double* vals = reinterpret_cast<double*>(smem_raw);
@@ -978,27 +967,25 @@ __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int c
     double own = 0.0;
     double hot = 0.0;
     bool hot_seen = false;
-    uint32_t slots[(MAXW + 1) / 2] = {};
-    uint32_t owned;
+    uint32_t cnt = 0;  // this warp's claims
     insert_block_range<MAXW, RULE, NT>(L, s, 0, d, v, cv, keys, vals, tv - 1, own, hot,
-                                   hot_seen, slots, owned);
+                                       hot_seen, list, cnt);
     // every warp adds its share of the own community's weight to that
     // community's slot (FP64 sums of FP32 weights are exact in any order),
     // so no block-wide sum is needed before the table is complete; the
     // warp whose add put the key in owns the candidate
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     hot = group_sum<32>(hot);
-    uint32_t hot_slot = kEmptyKey;
+    bool claimed = false;
     if (__any_sync(kFull, hot_seen) && lane == 0) {
-      bool claimed;
       const uint32_t slot = table_claim(keys, tv - 1, cv, L.sc, claimed);
       atomicAdd(&vals[slot], hot);
-      if (claimed) hot_slot = slot;
+      if (claimed) list[cnt] = (uint16_t)slot;
     }
+    cnt += __any_sync(kFull, claimed) ? 1u : 0u;
     if (RULE == LV_RULE_CUDA_I) own = group_sum<32>(own);
     __syncthreads();  // (A) the table is complete
-    K best = eval_owned<PREC, MAXW>(L, g, keys, vals, slots, owned, K{});
-    if (hot_slot != kEmptyKey) best = eval_own_slot<PREC>(L, g, keys, vals, hot_slot, best);
+    K best = eval_claims<PREC>(L, g, keys, vals, list, cnt);
     best = group_max<32>(best);
     if (lane == 0) {  // written after (A): thread 0 read the last ones before it
       red_best[wib] = best;
@@ -1029,7 +1016,8 @@ __global__ void __launch_bounds__(kThreads, kBlockPerSM)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ typename BestOf<ModeOf<MODE>::kPrec>::T red_best[kWarps];
   __shared__ double red_own[kWarps];
-  block_body<MODE>(D, cls, blockIdx.x, gridDim.x, smem_raw, red_best, red_own, io);
+  __shared__ uint16_t claims[kWarps * claim_list(kHubSmemMaxDeg, kThreads)];
+  block_body<MODE>(D, cls, blockIdx.x, gridDim.x, smem_raw, red_best, red_own, claims, io);
 }
 
 // deg <= 319 (KV_WARP512): a block of four warps per vertex, 512-slot table.
@@ -1048,8 +1036,9 @@ __global__ void __launch_bounds__(kTeamThreads, kTeamPerSM)
   __shared__ __align__(16) unsigned char smem_raw[kTeamSlots * kSlotBytes];
   __shared__ typename BestOf<ModeOf<MODE>::kPrec>::T red_best[kTeamThreads / 32];
   __shared__ double red_own[kTeamThreads / 32];
+  __shared__ uint16_t claims[kTeamThreads / 32 * claim_list(319, kTeamThreads)];
   block_body<MODE, kTeamThreads, kTeamSlots, 319>(D, cls, blockIdx.x, gridDim.x, smem_raw,
-                                                  red_best, red_own, io);
+                                                  red_best, red_own, claims, io);
 }
 
 // deg > 2048 (hubs).  The neighbour communities of a hub are split into P
@@ -2093,7 +2082,8 @@ __device__ __noinline__ void block_phase(const PassDesc* __restrict__ D, int cls
                                          uint32_t nblk, unsigned char* smem,
                                          typename BestOf<ModeOf<MODE>::kPrec>::T* red_best,
                                          double* red_d, StepIO io) {
-  block_body<MODE>(D, cls, bid, nblk, smem, red_best, red_d, io);
+  __shared__ uint16_t claims[kWarps * claim_list(kHubSmemMaxDeg, kThreads)];
+  block_body<MODE>(D, cls, bid, nblk, smem, red_best, red_d, claims, io);
 }
 template <int MODE>
 __device__ __noinline__ void split_phase(const PassDesc* __restrict__ D, uint32_t bid,

@@ -30,7 +30,7 @@ constexpr uint32_t kSmallWarpMerge = 128;  // entries of a community merged by a
 // row offsets, this block's class lists and proposals; what is left up to
 // kSmallSmem holds entries of its rows (8 bytes each).
 constexpr uint32_t kSmallArena = 4096u * (uint32_t)kSlotBytes;
-constexpr uint32_t kSmallSmem = 220u * 1024;
+constexpr uint32_t kSmallSmem = 216u * 1024;
 __host__ __device__ constexpr uint32_t small_own(uint32_t cap, uint32_t ctas) {
   return (cap + ctas - 1) / ctas;
 }
@@ -263,7 +263,8 @@ template <int MODE>
 __device__ __noinline__ void small_block(const PassDesc* D, int cls, unsigned char* smem) {
   __shared__ typename BestOf<ModeOf<MODE>::kPrec>::T rb[kSmallWarps];
   __shared__ double ro[kSmallWarps];
-  block_body<MODE, kSmallThreads>(D, cls, 0, 1, smem, rb, ro);
+  __shared__ uint16_t claims[kSmallWarps * claim_list(kHubSmemMaxDeg, kSmallThreads)];
+  block_body<MODE, kSmallThreads>(D, cls, 0, 1, smem, rb, ro, claims);
 }
 
 // One vertex's move into this block's copy of the state.  The lanes moving
