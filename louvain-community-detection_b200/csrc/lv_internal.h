@@ -112,6 +112,10 @@ struct LevelScalars {
   // intra-community weight from those rows only
   unsigned long long moved_acc;
   uint32_t inc_next;
+  // level init: an entry's weight is not a whole number >= 0; all are, and
+  // their total is below 2^31 (the move kernels add in 32-bit integers)
+  uint32_t frac;
+  uint32_t whole;
 };
 
 // Stop rule evaluated by the modularity sweep's last block when the pass

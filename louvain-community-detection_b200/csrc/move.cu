@@ -334,13 +334,30 @@ __device__ __forceinline__ uint32_t table_claim(uint32_t* keys, uint32_t mask, u
   return 0;
 }
 
+// Type of a table's sums: FP64 (exact for FP32 weights in any order), or
+// 32-bit integers on a level whose weights are all whole numbers of a total
+// below 2^31 (LevelScalars::whole; unweighted graphs and their contractions):
+// the same sums, added by the shared memory's own integer adder where an FP64
+// add is a loop of load, add and compare-and-swap.
+template <class S>
+__device__ __forceinline__ S to_sum(float w) {
+  return (S)w;
+}
+__device__ __forceinline__ double warp_total(double x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
+  return x;
+}
+__device__ __forceinline__ uint32_t warp_total(uint32_t x) { return __reduce_add_sync(kFull, x); }
+
 // Adds each lane's (key, w) to a shared table, the lanes holding the same
 // key as the wave's first entry summed with shuffles into one atomic: in
 // late passes a hub's neighbours crowd into a few communities, and
 // hundreds of threads looping on one slot's FP64 compare-and-swap made the
 // merge slower pass after pass.  A wave of distinct keys pays two ballots.
-__device__ __forceinline__ void table_add_wave(uint32_t* keys, double* vals, uint32_t mask,
-                                               bool has, uint32_t key, double w,
+template <class S>
+__device__ __forceinline__ void table_add_wave(uint32_t* keys, S* vals, uint32_t mask,
+                                               bool has, uint32_t key, S w,
                                                LevelScalars* sc) {
   const int lane = threadIdx.x & 31;
   const unsigned hm = __ballot_sync(0xffffffffu, has);
@@ -349,11 +366,9 @@ __device__ __forceinline__ void table_add_wave(uint32_t* keys, double* vals, uin
   const uint32_t kl = __shfl_sync(0xffffffffu, key, lead);
   const unsigned m = __ballot_sync(0xffffffffu, has && key == kl);
   if (__popc(m) > 1) {  // warp-uniform
-    double x = (m >> lane & 1u) ? w : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == lead) atomicAdd(&vals[table_insert(keys, mask, kl, sc)], x);
-    if (m >> lane & 1u) return;
+    const S x = warp_total((m >> lane & 1u) ? w : S(0));
+    if (lane == lead) w = x;
+    else if (m >> lane & 1u) has = false;
   }
   if (has) atomicAdd(&vals[table_insert(keys, mask, key, sc)], w);
 }
@@ -592,9 +607,9 @@ __global__ void __launch_bounds__(kThreads, kSmallPerSM)
 // threads from tid, four slots per thread at a time so the gathers
 // overlap); each thread empties the taken slots it read, leaving the table
 // clean.
-template <int PREC, bool kAllSizes = false>
+template <int PREC, bool kAllSizes = false, class S = double>
 __device__ __forceinline__ typename BestOf<PREC>::T scan_table_and_clear(
-    const LevelView& L, const GainCtx& g, uint32_t* keys, double* vals,
+    const LevelView& L, const GainCtx& g, uint32_t* keys, S* vals,
     uint32_t tv, uint32_t tid, uint32_t nthr) {
   typename BestOf<PREC>::T best{};
 #pragma unroll 1
@@ -605,7 +620,7 @@ __device__ __forceinline__ typename BestOf<PREC>::T scan_table_and_clear(
     for (int q = 0; q < 4; q++) {
       const uint32_t i = i0 + q * nthr;
       c[q] = i < tv ? keys[i] : kEmptyKey;
-      ec[q] = c[q] != kEmptyKey ? vals[i] : 0.0;
+      ec[q] = c[q] != kEmptyKey ? (double)vals[i] : 0.0;
     }
 #pragma unroll
     for (int q = 0; q < 4; q++) {
@@ -623,7 +638,7 @@ __device__ __forceinline__ typename BestOf<PREC>::T scan_table_and_clear(
         best = best_max(best, candidate_loaded<PREC>(g, c[q], ec[q], szc[q], ac[q]));
         const uint32_t i = i0 + q * nthr;
         keys[i] = kEmptyKey;
-        vals[i] = 0.0;
+        vals[i] = S(0);
       }
     }
   }
@@ -682,10 +697,10 @@ __device__ __forceinline__ void load_row_vec(const LevelView& L, uint64_t s, uin
 // its empty slots.  (With a thread evaluating its own claims, a warp walked
 // all its insert rounds for the one or two candidates a lane has once
 // communities have formed: 5.5-7 of 21 thousand cycles a vertex.)
-template <int PREC>
+template <int PREC, class S>
 __device__ __forceinline__ typename BestOf<PREC>::T eval_claims(const LevelView& L,
                                                                 const GainCtx& g, uint32_t* keys,
-                                                                double* vals,
+                                                                S* vals,
                                                                 const uint16_t* list,
                                                                 uint32_t cnt) {
   typename BestOf<PREC>::T best{};
@@ -698,7 +713,7 @@ __device__ __forceinline__ typename BestOf<PREC>::T eval_claims(const LevelView&
       if (i0 + 32 * q < cnt) {
         slot[q] = list[i0 + 32 * q];
         c[q] = keys[slot[q]];
-        ec[q] = vals[slot[q]];
+        ec[q] = (double)vals[slot[q]];
         szc[q] = candidate_size(L, g, c[q]);
         ac[q] = L.tot[c[q]];
       }
@@ -708,7 +723,7 @@ __device__ __forceinline__ typename BestOf<PREC>::T eval_claims(const LevelView&
       if (i0 + 32 * q < cnt) {
         best = best_max(best, candidate_loaded<PREC>(g, c[q], ec[q], szc[q], ac[q]));
         keys[slot[q]] = kEmptyKey;
-        vals[slot[q]] = 0.0;
+        vals[slot[q]] = S(0);
       }
     }
   }
@@ -864,13 +879,13 @@ __device__ __forceinline__ double block_sum(double x, double* red) {
 // registers -- every load issued before any is used -- then inserts them
 // into a table (clear it before, synchronise after).  The slots of the keys
 // this warp put in go to its list (eval_claims), `cnt` of them.
-template <int MAXW, int RULE, int NT>
+template <int MAXW, int RULE, int NT, class S>
 __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t s,
                                                    uint64_t lo, uint64_t end,
                                                    uint32_t v, uint32_t cv,
-                                                   uint32_t* keys, double* vals,
+                                                   uint32_t* keys, S* vals,
                                                    uint32_t mask, double& own,
-                                                   double& hot, bool& hot_seen,
+                                                   S& hot, bool& hot_seen,
                                                    uint16_t* list, uint32_t& cnt) {
   uint32_t cu[MAXW];
   float wt[MAXW];
@@ -900,7 +915,7 @@ __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t 
     const bool is_hot = has && cu[k] == cv;
     const bool ins = has && !is_hot;
     if (is_hot) {
-      hot += (double)wt[k];
+      hot += to_sum<S>(wt[k]);
       hot_seen = true;
       if (RULE == LV_RULE_CUDA_I && !(self_mask >> k & 1u)) own += (double)wt[k];
     }
@@ -908,7 +923,7 @@ __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t 
     uint32_t slot = 0;
     if (ins) {
       slot = table_claim(keys, mask, cu[k], L.sc, claimed);
-      atomicAdd(&vals[slot], (double)wt[k]);
+      atomicAdd(&vals[slot], to_sum<S>(wt[k]));
     }
     const unsigned cb = __ballot_sync(kFull, claimed);
     if (claimed) list[cnt + __popc(cb & lt)] = (uint16_t)slot;
@@ -921,12 +936,12 @@ __device__ __forceinline__ void insert_block_range(const LevelView& L, uint64_t 
 __host__ __device__ constexpr int claim_list(int maxdeg, int nt) { return (maxdeg + nt - 1) / nt * 32 + 2; }
 
 // A block of NT threads per vertex of at most MAXDEG entries, T-slot table.
-template <int MODE, int NT = kThreads, int T = kHubSmemSlots, int MAXDEG = (int)kHubSmemMaxDeg>
-__device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int cls, uint32_t bid,
+template <int MODE, class S, int NT, int T, int MAXDEG>
+__device__ __forceinline__ void block_rows(const PassDesc* __restrict__ D, int cls, uint32_t bid,
                                            uint32_t nblk, unsigned char* smem_raw,
                                            typename BestOf<ModeOf<MODE>::kPrec>::T* red_best,
                                            double* red_own, uint16_t* claims,
-                                           const StepIO io = StepIO{}) {
+                                           const StepIO io) {
   constexpr int RULE = ModeOf<MODE>::kRule, PREC = ModeOf<MODE>::kPrec;
   using K = typename BestOf<PREC>::T;
   const LevelView L = step_view(D, io);
@@ -936,7 +951,7 @@ __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int c
   uint16_t* list = claims + (threadIdx.x >> 5) * claim_list(MAXDEG, NT);
   const uint32_t count = D->act_cnt ? D->act_cnt[cls] : D->A.P.cls_start[cls + 1] - s0;
   constexpr int MAXW = (MAXDEG + NT - 1) / NT;
-  double* vals = reinterpret_cast<double*>(smem_raw);
+  S* vals = reinterpret_cast<S*>(smem_raw);
   uint32_t* keys = reinterpret_cast<uint32_t*>(smem_raw + sizeof(double) * T);
   uint32_t clean = 0;  // leading table slots known to be empty
   // the first vertex's id, row and community are on their way while the
@@ -958,14 +973,14 @@ __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int c
     if (tv > clean) {  // block-uniform; the scan empties what a row used
       for (uint32_t i = clean + threadIdx.x; i < tv; i += NT) {
         keys[i] = kEmptyKey;
-        vals[i] = 0.0;
+        vals[i] = S(0);
       }
       clean = tv;
       __syncthreads();
     }
     const GainCtx g = make_ctx<PREC>(L, v, cv);
     double own = 0.0;
-    double hot = 0.0;
+    S hot = S(0);
     bool hot_seen = false;
     uint32_t cnt = 0;  // this warp's claims
     insert_block_range<MAXW, RULE, NT>(L, s, 0, d, v, cv, keys, vals, tv - 1, own, hot,
@@ -975,7 +990,7 @@ __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int c
     // so no block-wide sum is needed before the table is complete; the
     // warp whose add put the key in owns the candidate
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    hot = group_sum<32>(hot);
+    hot = warp_total(hot);
     bool claimed = false;
     if (__any_sync(kFull, hot_seen) && lane == 0) {
       const uint32_t slot = table_claim(keys, tv - 1, cv, L.sc, claimed);
@@ -1007,6 +1022,20 @@ __device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int c
     // rewritten only after the next (A), which thread 0 reaches after it
     // has read them
   }
+}
+
+template <int MODE, int NT = kThreads, int T = kHubSmemSlots, int MAXDEG = (int)kHubSmemMaxDeg>
+__device__ __forceinline__ void block_body(const PassDesc* __restrict__ D, int cls, uint32_t bid,
+                                           uint32_t nblk, unsigned char* smem_raw,
+                                           typename BestOf<ModeOf<MODE>::kPrec>::T* red_best,
+                                           double* red_own, uint16_t* claims,
+                                           const StepIO io = StepIO{}) {
+  if (D->L.sc->whole)
+    block_rows<MODE, uint32_t, NT, T, MAXDEG>(D, cls, bid, nblk, smem_raw, red_best, red_own,
+                                              claims, io);
+  else
+    block_rows<MODE, double, NT, T, MAXDEG>(D, cls, bid, nblk, smem_raw, red_best, red_own,
+                                            claims, io);
 }
 
 // 319 < deg <= 2048: one block per vertex, shared 4096-slot table.
@@ -1189,12 +1218,12 @@ __global__ void __launch_bounds__(kThreads, kSplitPerSM)
   split_body<MODE>(D, blockIdx.x, gridDim.x, cnt, wsum, red, io);
 }
 
-template <int MODE>
-__device__ __forceinline__ void merge_body(const PassDesc* __restrict__ D, uint32_t bid,
+template <int MODE, class S>
+__device__ __forceinline__ void merge_units(const PassDesc* __restrict__ D, uint32_t bid,
                                            uint32_t nblk, unsigned char* smem_raw,
                                            typename BestOf<ModeOf<MODE>::kPrec>::T* red_best,
                                            uint32_t* seg_a, uint32_t* seg_pre, uint32_t* wsum,
-                                           const StepIO io = StepIO{}) {
+                                           const StepIO io) {
   constexpr int PREC = ModeOf<MODE>::kPrec;
   using K = typename BestOf<PREC>::T;
   const LevelView L = step_view(D, io);
@@ -1202,11 +1231,11 @@ __device__ __forceinline__ void merge_body(const PassDesc* __restrict__ D, uint3
   const HubArena H = D->H;
   const uint32_t units = H.units;
   constexpr int T = kHubPartSlots;
-  double* vals = reinterpret_cast<double*>(smem_raw);
+  S* vals = reinterpret_cast<S*>(smem_raw);
   uint32_t* keys = reinterpret_cast<uint32_t*>(smem_raw + sizeof(double) * T);
   for (uint32_t i = threadIdx.x; i < T; i += kThreads) {
     keys[i] = kEmptyKey;
-    vals[i] = 0.0;
+    vals[i] = S(0);
   }
   __syncthreads();
   for (uint32_t u = bid; u < units; u += nblk) {
@@ -1247,7 +1276,7 @@ __device__ __forceinline__ void merge_body(const PassDesc* __restrict__ D, uint3
           c = cw.x;
           w = __uint_as_float(cw.y);
         }
-        table_add_wave(keys, vals, T - 1, has, c, (double)w, L.sc);
+        table_add_wave(keys, vals, T - 1, has, c, to_sum<S>(w), L.sc);
       }
       __syncthreads();  // seg_a / seg_pre are refilled
     }
@@ -1264,6 +1293,18 @@ __device__ __forceinline__ void merge_body(const PassDesc* __restrict__ D, uint3
     }
     __syncthreads();
   }
+}
+
+template <int MODE>
+__device__ __forceinline__ void merge_body(const PassDesc* __restrict__ D, uint32_t bid,
+                                           uint32_t nblk, unsigned char* smem_raw,
+                                           typename BestOf<ModeOf<MODE>::kPrec>::T* red_best,
+                                           uint32_t* seg_a, uint32_t* seg_pre, uint32_t* wsum,
+                                           const StepIO io = StepIO{}) {
+  if (D->L.sc->whole)
+    merge_units<MODE, uint32_t>(D, bid, nblk, smem_raw, red_best, seg_a, seg_pre, wsum, io);
+  else
+    merge_units<MODE, double>(D, bid, nblk, smem_raw, red_best, seg_a, seg_pre, wsum, io);
 }
 
 template <int MODE>
@@ -1354,6 +1395,7 @@ __global__ void __launch_bounds__(kThreads, kSweepPerSM)
 // consecutive, and graphs are runs of every class list).
 struct RowSumOp {
   double m = 0.0, self = 0.0, asq = 0.0;
+  bool frac = false;  // an entry's weight is not a whole number
   uint32_t graph = kNoGraph;
   __device__ bool row(const LevelView&, uint32_t) const { return true; }
   __device__ uint32_t ctx(const LevelView& L, uint32_t v) {
@@ -1368,6 +1410,7 @@ struct RowSumOp {
   }
   __device__ double edge(const LevelView&, uint32_t v, uint32_t u, float w) {
     if (u == v) self += (double)w;
+    frac |= !(w >= 0.0f && w == truncf(w));
     return (double)w;
   }
   __device__ void vertex(const LevelView& L, uint32_t v, double sum) {
@@ -1644,6 +1687,7 @@ __global__ void __launch_bounds__(kThreads)
       }
     }
   }
+  if (__syncthreads_or(op.frac) && threadIdx.x == 0) atomicOr(&L.sc->frac, 1u);
   if (!publish_and_check_last(op.m, op.self, op.asq, A, L.sc, gridDim.x)) return;
   const Sums3 all = sum_partials(A, gridDim.x, red);
   // hubs: finalise their row sums in index order
@@ -1679,6 +1723,8 @@ __global__ void __launch_bounds__(kThreads)
     L.sc->asq = sq;
     L.sc->q = (m64 > 0.0) ? (all.b / (2.0 * m64)) - (sq / (4.0 * m64 * m64)) : 0.0;
     L.sc->done_blocks = 0u;
+    L.sc->whole = !__ldcg(&L.sc->frac) && m64 < 1073741824.0;
+    L.sc->frac = 0u;
   }
   // batched form: every graph's own (the union's above are unused)
   if (L.gid) {

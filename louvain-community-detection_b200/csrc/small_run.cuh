@@ -264,7 +264,8 @@ __device__ __noinline__ void small_block(const PassDesc* D, int cls, unsigned ch
   __shared__ typename BestOf<ModeOf<MODE>::kPrec>::T rb[kSmallWarps];
   __shared__ double ro[kSmallWarps];
   __shared__ uint16_t claims[kSmallWarps * claim_list(kHubSmemMaxDeg, kSmallThreads)];
-  block_body<MODE, kSmallThreads>(D, cls, 0, 1, smem, rb, ro, claims);
+  block_rows<MODE, double, kSmallThreads, kHubSmemSlots, (int)kHubSmemMaxDeg>(
+      D, cls, 0, 1, smem, rb, ro, claims, StepIO{});
 }
 
 // One vertex's move into this block's copy of the state.  The lanes moving
