@@ -89,6 +89,8 @@ __device__ __forceinline__ double warp_sum(double x) {
   return x;
 }
 
+__device__ __forceinline__ uint32_t warp_sum(uint32_t x) { return __reduce_add_sync(kFull, x); }
+
 struct Ctx {
   const uint64_t* off;
   const uint32_t* col;
@@ -103,6 +105,7 @@ struct Ctx {
   float* tw;
   uint64_t* new_deg;
   uint32_t* err;
+  const uint32_t* whole;  // the level's LevelScalars::whole
 };
 
 // flag_id[c] = comm_sz[c] > 0 ; mem_off[c] = comm_sz[c]  (scanned after)
@@ -256,13 +259,13 @@ __global__ void g_fill_kernel(const uint32_t* __restrict__ counts,
 }
 
 // Class W: one warp per community, flattened member edges, 256-slot table.
-__global__ void __launch_bounds__(kThreads)
-    merge_warp_kernel(Ctx C, const uint32_t* list, uint32_t count) {
-  __shared__ double vals_sm[kWarps][kWarpSlots];
-  __shared__ uint32_t keys_sm[kWarps][kWarpSlots];
+// S: type of a table's sums -- FP64, or 32-bit integers on a level of whole
+// weights (LevelScalars::whole; exact either way), which shared memory adds
+// by itself where an FP64 add is a loop around a compare-and-swap.
+template <class S>
+__device__ __forceinline__ void merge_warp_rows(const Ctx& C, const uint32_t* list,
+                                                uint32_t count, S* vals, uint32_t* keys) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  double* vals = vals_sm[wib];
-  uint32_t* keys = keys_sm[wib];
   for (uint32_t idx = blockIdx.x * kWarps + wib; idx < count;
        idx += gridDim.x * kWarps) {
     const uint32_t cn = list[idx];
@@ -274,12 +277,12 @@ __global__ void __launch_bounds__(kThreads)
     const uint32_t mask = tv - 1;
     for (uint32_t i = lane; i < tv; i += 32) {
       keys[i] = kEmptyKey;
-      vals[i] = 0.0;
+      vals[i] = S(0);
     }
     __syncwarp();
     // edges into the community itself (most of them, once the moves have
     // converged) are summed in registers instead of one contended slot
-    double hot_acc = 0.0;
+    S hot_acc = S(0);
     bool hot_seen = false;
     for (uint32_t mb = 0; mb < msz; mb += 32) {
       const uint32_t mi = mb + lane;
@@ -326,10 +329,10 @@ __global__ void __launch_bounds__(kThreads)
       for (int k = 0; k < kWaves; k++) {
         if (key[k] == kEmptyKey) continue;
         if (key[k] == cn) {  // intra-community edge: the new self-loop
-          hot_acc += (double)wt[k];
+          hot_acc += (S)wt[k];
           hot_seen = true;
         } else {  // every lane inserts its own entry: equal keys meet in the CAS
-          atomicAdd(&vals[table_insert(keys, mask, key[k], C.err)], (double)wt[k]);
+          atomicAdd(&vals[table_insert(keys, mask, key[k], C.err)], (S)wt[k]);
         }
       }
     }
@@ -356,6 +359,17 @@ __global__ void __launch_bounds__(kThreads)
     if (lane == 0) C.new_deg[cn] = cnt;
     __syncwarp();
   }
+}
+
+__global__ void __launch_bounds__(kThreads)
+    merge_warp_kernel(Ctx C, const uint32_t* list, uint32_t count) {
+  __shared__ double vals_sm[kWarps][kWarpSlots];
+  __shared__ uint32_t keys_sm[kWarps][kWarpSlots];
+  const int wib = threadIdx.x >> 5;
+  if (*C.whole)
+    merge_warp_rows(C, list, count, reinterpret_cast<uint32_t*>(vals_sm[wib]), keys_sm[wib]);
+  else
+    merge_warp_rows(C, list, count, vals_sm[wib], keys_sm[wib]);
 }
 
 template <int NT = kThreads>
@@ -388,15 +402,15 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t* sm,
 
 // Inserts positions [lo, hi) of a community's flattened edge range into a
 // table; members are staged through shared memory NT at a time.
-template <int NT = kThreads>
+template <int NT = kThreads, class S>
 __device__ __forceinline__ void insert_range(const Ctx& C, uint32_t m0,
                                              uint32_t msz, uint64_t seg,
                                              uint64_t total, uint64_t lo,
                                              uint64_t hi, uint32_t* keys,
-                                             double* vals, uint32_t mask,
+                                             S* vals, uint32_t mask,
                                              uint64_t* s_start,
                                              uint64_t* s_off, uint32_t hot,
-                                             double& hot_acc, bool& hot_seen) {
+                                             S& hot_acc, bool& hot_seen) {
   // first member whose range contains lo: largest k with start_k <= lo
   __shared__ uint32_t s_k;
   if (threadIdx.x == 0) {
@@ -453,10 +467,10 @@ __device__ __forceinline__ void insert_range(const Ctx& C, uint32_t m0,
       for (int k = 0; k < kWaves; k++) {
         if (key[k] == kEmptyKey) continue;
         if (key[k] == hot) {
-          hot_acc += (double)wt[k];
+          hot_acc += (S)wt[k];
           hot_seen = true;
         } else {
-          atomicAdd(&vals[table_insert(keys, mask, key[k], C.err)], (double)wt[k]);
+          atomicAdd(&vals[table_insert(keys, mask, key[k], C.err)], (S)wt[k]);
         }
       }
     }
@@ -469,15 +483,14 @@ __device__ __forceinline__ void insert_range(const Ctx& C, uint32_t m0,
 
 // Classes B (SLOTS = 2048: <= 1024 entries) and B2 (8192: <= 4096): one
 // block per community, shared table of up to SLOTS slots.
-template <int SLOTS, int NT>
-__global__ void __launch_bounds__(NT)
-    merge_block_kernel(Ctx C, const uint32_t* list, uint32_t count) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* vals = reinterpret_cast<double*>(smem_raw);
+template <int SLOTS, int NT, class S>
+__device__ __forceinline__ void merge_block_rows(const Ctx& C, const uint32_t* list,
+                                                 uint32_t count, unsigned char* smem_raw,
+                                                 uint32_t* scan_sm) {
+  S* vals = reinterpret_cast<S*>(smem_raw);
   uint64_t* s_start = reinterpret_cast<uint64_t*>(smem_raw + SLOTS * 8);
   uint64_t* s_off = s_start + NT;
   uint32_t* keys = reinterpret_cast<uint32_t*>(smem_raw + SLOTS * 8 + NT * 16);
-  __shared__ uint32_t scan_sm[NT / 32 + 1];
   for (uint32_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
     const uint32_t cn = list[idx];
     const uint32_t c = C.comm_list[cn];
@@ -488,10 +501,10 @@ __global__ void __launch_bounds__(NT)
     const uint32_t tv = max(table_size_for((uint32_t)total, SLOTS), (uint32_t)NT);
     for (uint32_t i = threadIdx.x; i < tv; i += NT) {
       keys[i] = kEmptyKey;
-      vals[i] = 0.0;
+      vals[i] = S(0);
     }
     __syncthreads();
-    double hot_acc = 0.0;
+    S hot_acc = S(0);
     bool hot_seen = false;
     insert_range<NT>(C, m0, msz, seg, total, 0, total, keys, vals, tv - 1, s_start, s_off, cn,
                  hot_acc, hot_seen);
@@ -519,6 +532,17 @@ __global__ void __launch_bounds__(NT)
     if (threadIdx.x == 0) C.new_deg[cn] = tot;
     __syncthreads();
   }
+}
+
+template <int SLOTS, int NT>
+__global__ void __launch_bounds__(NT)
+    merge_block_kernel(Ctx C, const uint32_t* list, uint32_t count) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint32_t scan_sm[NT / 32 + 1];
+  if (*C.whole)
+    merge_block_rows<SLOTS, NT, uint32_t>(C, list, count, smem_raw, scan_sm);
+  else
+    merge_block_rows<SLOTS, NT, double>(C, list, count, smem_raw, scan_sm);
 }
 
 struct GArgs {
@@ -908,6 +932,7 @@ cudaError_t contract_back(const LevelView& L, uint64_t nnz, ContractBuffers& B,
   C.tw = B.tw;
   C.new_deg = B.new_deg;
   C.err = &L.sc->error;
+  C.whole = &L.sc->whole;
 
   if (cntW) {
     (count_launches(1), merge_warp_kernel<<<gridcap((cntW + kWarps - 1) / kWarps, 4), kThreads, 0, st>>>(

@@ -734,11 +734,11 @@ __device__ __forceinline__ typename BestOf<PREC>::T eval_claims(const LevelView&
 // row's loads (at most MAXW waves of 32) are issued before any insertion,
 // so a vertex costs one memory latency chain instead of one per wave.  nw:
 // the block's warps that have a table (its first ones).
-template <int T, int MAXW, int MODE, bool COHERENT = false>
-__device__ __forceinline__ void warp_body(const PassDesc* __restrict__ D, int cls, uint32_t bid,
+template <int T, int MAXW, int MODE, class S, bool COHERENT>
+__device__ __forceinline__ void warp_rows(const PassDesc* __restrict__ D, int cls, uint32_t bid,
                                           uint32_t nblk, unsigned char* smem_raw,
-                                          const StepIO io = StepIO{},
-                                          const uint32_t nw = kWarps) {
+                                          const StepIO io,
+                                          const uint32_t nw) {
   constexpr int RULE = ModeOf<MODE>::kRule, PREC = ModeOf<MODE>::kPrec;
   const LevelView L = step_view(D, io);
   reapply_prev_step(D, io, bid, nblk);
@@ -748,7 +748,7 @@ __device__ __forceinline__ void warp_body(const PassDesc* __restrict__ D, int cl
   uint32_t* __restrict__ prop = D->prop + s0;
   const uint32_t count = D->act_cnt ? D->act_cnt[cls] : D->A.P.cls_start[cls + 1] - s0;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  double* vals = reinterpret_cast<double*>(smem_raw) + wib * T;
+  S* vals = reinterpret_cast<S*>(smem_raw) + wib * T;
   uint32_t* keys = reinterpret_cast<uint32_t*>(smem_raw + sizeof(double) * T * nw) + wib * T;
   uint32_t clean = 0;  // leading table slots known to be empty
   if (COHERENT && (uint32_t)wib >= nw) return;
@@ -766,7 +766,7 @@ __device__ __forceinline__ void warp_body(const PassDesc* __restrict__ D, int cl
     if (tv > clean) {  // warp-uniform; the scan empties what a row used
       for (uint32_t i = clean + lane; i < tv; i += 32) {
         keys[i] = kEmptyKey;
-        vals[i] = 0.0;
+        vals[i] = S(0);
       }
       clean = tv;
       __syncwarp();
@@ -806,7 +806,8 @@ __device__ __forceinline__ void warp_body(const PassDesc* __restrict__ D, int cl
       if (has && cu[i] == v) self_mask |= 1u << i;
       cu[i] = has ? L.comm[cu[i]] : kEmptyKey;  // kEmptyKey: no entry
     }
-    double own = 0.0, hot = 0.0;
+    double own = 0.0;
+    S hot = S(0);
     bool hot_seen = false;
 #pragma unroll
     for (int i = 0; i < NE; i++) {
@@ -817,14 +818,14 @@ __device__ __forceinline__ void warp_body(const PassDesc* __restrict__ D, int cl
       const bool is_hot = has && cu[i] == cv;
       const bool ins = has && !is_hot;
       if (is_hot) {
-        hot += (double)wt[i];
+        hot += to_sum<S>(wt[i]);
         hot_seen = true;
         if (RULE == LV_RULE_CUDA_I && !(self_mask >> i & 1u)) own += (double)wt[i];
       }
       // every lane inserts its own entry: equal keys meet in the CAS
-      if (ins) atomicAdd(&vals[table_insert(keys, tv - 1, cu[i], L.sc)], (double)wt[i]);
+      if (ins) atomicAdd(&vals[table_insert(keys, tv - 1, cu[i], L.sc)], to_sum<S>(wt[i]));
     }
-    hot = group_sum<32>(hot);
+    hot = warp_total(hot);
     if (__any_sync(kFull, hot_seen) && lane == 0) {
       const uint32_t slot = table_insert(keys, tv - 1, cv, L.sc);
       vals[slot] += hot;
@@ -839,6 +840,17 @@ __device__ __forceinline__ void warp_body(const PassDesc* __restrict__ D, int cl
     if (lane == 0) record_decision(D, io, &prop[vidx], v, g, decide<RULE>(best, own, g));
     __syncwarp();
   }
+}
+
+template <int T, int MAXW, int MODE, bool COHERENT = false>
+__device__ __forceinline__ void warp_body(const PassDesc* __restrict__ D, int cls, uint32_t bid,
+                                          uint32_t nblk, unsigned char* smem_raw,
+                                          const StepIO io = StepIO{},
+                                          const uint32_t nw = kWarps) {
+  if (D->L.sc->whole)
+    warp_rows<T, MAXW, MODE, uint32_t, COHERENT>(D, cls, bid, nblk, smem_raw, io, nw);
+  else
+    warp_rows<T, MAXW, MODE, double, COHERENT>(D, cls, bid, nblk, smem_raw, io, nw);
 }
 
 template <int T, int MAXW, int MODE>

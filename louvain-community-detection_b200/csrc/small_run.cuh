@@ -257,7 +257,7 @@ __device__ __noinline__ void small_lanes(const PassDesc* D, int cls, unsigned ch
 template <int T, int MAXW, int MODE>
 __device__ __noinline__ void small_warp(const PassDesc* D, int cls, unsigned char* smem,
                                         uint32_t warps) {
-  warp_body<T, MAXW, MODE, true>(D, cls, 0, 1, smem, StepIO{}, warps);
+  warp_rows<T, MAXW, MODE, double, true>(D, cls, 0, 1, smem, StepIO{}, warps);
 }
 template <int MODE>
 __device__ __noinline__ void small_block(const PassDesc* D, int cls, unsigned char* smem) {
