@@ -254,6 +254,8 @@ __device__ __noinline__ void small_lanes(const PassDesc* D, int cls, unsigned ch
       D, cls, 0, 1, reinterpret_cast<double(*)[32]>(smem),
       reinterpret_cast<uint32_t(*)[64]>(smem + kSmallWarps * 32 * sizeof(double)));
 }
+// The table phases add in FP64 whatever the weights: a level of this size has
+// few rows for them.
 template <int T, int MAXW, int MODE>
 __device__ __noinline__ void small_warp(const PassDesc* D, int cls, unsigned char* smem,
                                         uint32_t warps) {
