@@ -428,12 +428,12 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t* sm,
 
 // Inserts positions [lo, hi) of a community's flattened edge range into a
 // table; members are staged through shared memory NT at a time.
-template <int NT = kThreads, class S>
+// Add: what an entry (key, weight) outside the community does.
+template <int NT = kThreads, class S, class Add>
 __device__ __forceinline__ void insert_range(const Ctx& C, uint32_t m0,
                                              uint32_t msz, uint64_t seg,
                                              uint64_t total, uint64_t lo,
-                                             uint64_t hi, uint32_t* keys,
-                                             S* vals, uint32_t mask,
+                                             uint64_t hi, Add add,
                                              uint64_t* s_start,
                                              uint64_t* s_off, uint32_t hot,
                                              S& hot_acc, bool& hot_seen) {
@@ -496,7 +496,7 @@ __device__ __forceinline__ void insert_range(const Ctx& C, uint32_t m0,
           hot_acc += (S)wt[k];
           hot_seen = true;
         } else {
-          atomicAdd(&vals[table_insert(keys, mask, key[k], C.err)], (S)wt[k]);
+          add(key[k], wt[k]);
         }
       }
     }
@@ -532,8 +532,11 @@ __device__ __forceinline__ void merge_block_rows(const Ctx& C, const uint32_t* l
     __syncthreads();
     S hot_acc = S(0);
     bool hot_seen = false;
-    insert_range<NT>(C, m0, msz, seg, total, 0, total, keys, vals, tv - 1, s_start, s_off, cn,
-                 hot_acc, hot_seen);
+    auto add = [&](uint32_t key, float w) {
+      atomicAdd(&vals[table_insert(keys, tv - 1, key, C.err)], (S)w);
+    };
+    insert_range<NT>(C, m0, msz, seg, total, 0, total, add, s_start, s_off, cn, hot_acc,
+                     hot_seen);
     // every warp adds its share of the new self-loop (FP64 sums of FP32
     // weights are exact in any order): no block-wide sum first
     hot_acc = warp_sum(hot_acc);
@@ -584,11 +587,25 @@ struct GArgs {
 };
 
 // Class G: blocks insert chunks of a community's flattened range into its
-// global table.
-__global__ void __launch_bounds__(kThreads)
-    merge_global_insert_kernel(Ctx C, GArgs G) {
-  __shared__ uint64_t s_start[kThreads];
-  __shared__ uint64_t s_off[kThreads];
+// global table.  The entries between two large communities all meet in one
+// address, which bounded the kernel, so a chunk's first keys (one a slot of a
+// small direct-mapped table) are summed in shared memory and added once;
+// the others go to the global table as they come: R-MAT 20's first level
+// 2,982 -> 391 us.  (A shared table for all of a chunk's keys, most of them
+// distinct, was slower than none.)  Communities of few chunks have no such
+// address and only pay the detour (LFR 1 M with it: 98 -> 180 us a level), so
+// it is for those of at least kGCacheMin entries.
+constexpr int kGCache = 512;
+constexpr uint64_t kGCacheMin = 128 * (uint64_t)kMergeChunk;
+template <class S>
+__device__ __forceinline__ void merge_global_rows(const Ctx& C, const GArgs& G,
+                                                  uint64_t* s_start, uint64_t* s_off,
+                                                  uint32_t* ckeys, S* cvals) {
+  for (uint32_t i = threadIdx.x; i < kGCache; i += kThreads) {
+    ckeys[i] = kEmptyKey;
+    cvals[i] = S(0);
+  }
+  __syncthreads();
   for (uint32_t b = blockIdx.x; b < G.nblocks; b += gridDim.x) {
     const uint32_t gi = G.blk_comm[b], ch = G.blk_chunk[b];
     const uint32_t cn = G.list[gi];
@@ -603,13 +620,46 @@ __global__ void __launch_bounds__(kThreads)
     const uint32_t mask = G.tab_size[gi] - 1;
     double hot_acc = 0.0;
     bool hot_seen = false;
-    insert_range(C, m0, msz, seg, total, lo, hi, keys, vals, mask, s_start, s_off, cn,
-                 hot_acc, hot_seen);
+    const bool cached = total >= kGCacheMin;  // block-uniform
+    auto add = [&](uint32_t key, float w) {
+      if (!cached) {
+        atomicAdd(&vals[table_insert(keys, mask, key, C.err)], (double)w);
+        return;
+      }
+      const uint32_t h = hash_slot(key, kGCache - 1);
+      uint32_t cur = ckeys[h];
+      if (cur == kEmptyKey) {
+        cur = atomicCAS(&ckeys[h], kEmptyKey, key);
+        if (cur == kEmptyKey) cur = key;
+      }
+      if (cur == key) atomicAdd(&cvals[h], (S)w);
+      else atomicAdd(&vals[table_insert(keys, mask, key, C.err)], (double)w);
+    };
+    insert_range(C, m0, msz, seg, total, lo, hi, add, s_start, s_off, cn, hot_acc, hot_seen);
+    // (its last barrier: every entry is in)
+    for (uint32_t i = threadIdx.x; cached && i < kGCache; i += kThreads) {
+      if (ckeys[i] == kEmptyKey) continue;
+      atomicAdd(&vals[table_insert(keys, mask, ckeys[i], C.err)], (double)cvals[i]);
+      ckeys[i] = kEmptyKey;
+      cvals[i] = S(0);
+    }
     hot_acc = warp_sum(hot_acc);  // per warp, as in merge_block_kernel
     if (__any_sync(kFull, hot_seen) && (threadIdx.x & 31) == 0)
       atomicAdd(&vals[table_insert(keys, mask, cn, C.err)], hot_acc);
     __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(kThreads)
+    merge_global_insert_kernel(Ctx C, GArgs G) {
+  __shared__ uint64_t s_start[kThreads];
+  __shared__ uint64_t s_off[kThreads];
+  __shared__ double cvals[kGCache];
+  __shared__ uint32_t ckeys[kGCache];
+  if (*C.whole)
+    merge_global_rows(C, G, s_start, s_off, ckeys, reinterpret_cast<uint32_t*>(cvals));
+  else
+    merge_global_rows(C, G, s_start, s_off, ckeys, cvals);
 }
 
 // Class G: blocks compact slices of the tables into the staging rows.
