@@ -113,7 +113,8 @@ struct LevelScalars {
   unsigned long long moved_acc;
   uint32_t inc_next;
   // level init: an entry's weight is not a whole number >= 0; all are, and
-  // their total is below 2^31 (the move kernels add in 32-bit integers)
+  // their total (a union: every graph's) is below 2^31 (the move and merge
+  // tables add in 32-bit integers)
   uint32_t frac;
   uint32_t whole;
 };

@@ -336,11 +336,12 @@ __device__ __forceinline__ uint32_t table_claim(uint32_t* keys, uint32_t mask, u
 
 // Type of a table's sums: FP64 (exact for FP32 weights in any order), or
 // 32-bit integers on a level whose weights are all whole numbers of a total
-// below 2^31 (LevelScalars::whole; unweighted graphs and their contractions),
-// so that no sum wraps: the same sums.  Shared memory adds integers by itself;
-// an FP64 add is a loop of load, add and compare-and-swap, on which lanes that
-// meet in one community serialise (R-MAT 20, FP64 gains: block kernel 525 ->
-// 295 us a launch, hub merge 345 -> 193, warp kernel 113 -> 108; R-MAT 24:
+// below 2^31 in every graph (LevelScalars::whole; unweighted graphs and their
+// contractions), so that no sum wraps: the same sums.  Shared memory adds
+// integers by itself; an FP64 add is a loop of load, add and compare-and-swap,
+// on which lanes that meet in one community serialise (R-MAT 20, FP64 gains:
+// block kernel 525 -> 295 us a launch, hub merge 345 -> 193, warp kernel
+// 113 -> 108; R-MAT 24:
 // 3,310 -> 2,380, 7,860 -> 6,220, 1,200 -> 1,150).
 template <class S>
 __device__ __forceinline__ S to_sum(float w) {
@@ -1663,6 +1664,10 @@ __device__ __forceinline__ void dispatch_units(const LevelView& L, const Dispatc
   }
 }
 
+// Half the total weight below which 32-bit sums of whole weights cannot wrap:
+// no sum exceeds the total, 2^31 (LevelScalars::whole).
+constexpr double kWholeMax = 1073741824.0;
+
 __global__ void __launch_bounds__(kThreads)
     level_init_kernel(LevelView L, DispatchArgs A, uint32_t* __restrict__ rowid,
                       uint32_t* __restrict__ comm_start) {
@@ -1729,6 +1734,7 @@ __global__ void __launch_bounds__(kThreads)
   // m and the modularity of the singleton partition: the self-loops are its
   // intra-community weight, the degrees its totals (its own sweep over the
   // entries took 1.3 ms of R-MAT 24's 8.5 ms set-up, 545 of 940 us on a batch)
+  bool fits = true;
   if (threadIdx.x == 0) {
     const double m64 = (all.a + hs) / 2.0;
     const float m = (float)m64;
@@ -1740,14 +1746,15 @@ __global__ void __launch_bounds__(kThreads)
     L.sc->asq = sq;
     L.sc->q = (m64 > 0.0) ? (all.b / (2.0 * m64)) - (sq / (4.0 * m64 * m64)) : 0.0;
     L.sc->done_blocks = 0u;
-    L.sc->whole = !__ldcg(&L.sc->frac) && m64 < 1073741824.0;
-    L.sc->frac = 0u;
+    if (!L.gid) fits = m64 < kWholeMax;
   }
-  // batched form: every graph's own (the union's above are unused)
+  // batched form: every graph's own.  The union's above hold only its hubs:
+  // the other rows' sums went to their graphs (RowSumOp::flush)
   if (L.gid) {
     for (uint32_t g = threadIdx.x; g < L.n_graphs; g += kThreads) {
       GraphState& gs = L.gs[g];
       const double m64 = __ldcg(&gs.m_acc) / 2.0;
+      fits &= m64 < kWholeMax;  // a table's sum is of one graph's entries
       const float m = (float)m64;
       gs.m64 = m64;
       gs.m = m;
@@ -1759,6 +1766,11 @@ __global__ void __launch_bounds__(kThreads)
       gs.intra_acc = 0.0;
       gs.asq_acc = 0.0;
     }
+  }
+  fits = __syncthreads_and(fits);
+  if (threadIdx.x == 0) {
+    L.sc->whole = fits && !__ldcg(&L.sc->frac);
+    L.sc->frac = 0u;
   }
 }
 
