@@ -376,7 +376,7 @@ struct lv_engine {
   // small-run kernel: its buffers (one allocation) and pinned result
   unsigned char* small_buf = nullptr;
   SmallRunResult* small_host = nullptr;
-  bool small_off = false;  // the device cannot run it
+  int small_ctas = -1;  // its cluster on this device (0: cannot run it; -1: not asked yet)
   DispatchPlan plan{};
   double q_last = 0.0;
   std::vector<lv_level_info> levels;
@@ -2138,7 +2138,7 @@ static uint64_t small_max_entries(const lv_engine* E) {
 // is the level before's then): the kernel refuses a level with too many.
 static bool small_eligible(const lv_engine* E) {
   return E->cfg.use_graphs && !E->profiling && !E->batch && !use_level_kernel(E) &&
-         !E->cfg.contract_sort && !E->cfg.apply_launch && !E->level_ready && !E->small_off &&
+         !E->cfg.contract_sort && !E->cfg.apply_launch && !E->level_ready && E->small_ctas &&
          E->n > 0 && E->n <= kSmallMaxN &&
          (E->agg_pending ? E->e <= kSmallPrevEntries || (uint64_t)E->n * E->n <= small_max_entries(E)
                          : E->e <= small_max_entries(E));
@@ -2151,6 +2151,8 @@ static lv_status small_run(lv_engine* E, float min_gain, bool move_only, bool* t
   *took = false;
   cudaStream_t st = E->st;
   constexpr size_t kIds = (size_t)kSmallMaxN * sizeof(uint32_t);
+  if (E->small_ctas < 0) E->small_ctas = small_run_cluster(engine_mode(E));
+  if (!E->small_ctas) return LV_OK;
   if (!E->small_buf) CU(dalloc(&E->small_buf, kIds + 256 + sizeof(SmallRunResult)));
   unsigned char* b = E->small_buf;
   SmallRunArgs a{};
@@ -2178,12 +2180,7 @@ static lv_status small_run(lv_engine* E, float min_gain, bool move_only, bool* t
   a.move_only = move_only ? 1u : 0u;
   const bool one = E->n <= kSmallOneMaxN &&
                    (E->agg_pending ? E->n <= kSmallOneVertices : E->e <= kSmallOneEntries);
-  const cudaError_t ce = launch_small_run(a, engine_mode(E), one, st);
-  if (ce == cudaErrorNotSupported) {
-    E->small_off = true;
-    return LV_OK;
-  }
-  CU(ce);
+  CU(launch_small_run(a, engine_mode(E), one ? 1u : (unsigned)E->small_ctas, st));
   SmallRunResult* R = E->small_host;
   CU(cudaMemcpyAsync(R, a.res, sizeof(SmallRunResult), cudaMemcpyDeviceToHost, st));
   CU(cudaMemcpyAsync(E->sc_host, E->sc, sizeof(LevelScalars), cudaMemcpyDeviceToHost, st));

@@ -554,10 +554,14 @@ struct SmallRunArgs {
   uint32_t max_passes, max_levels;  // levels this run may still do (0: no cap)
   uint32_t move_only;       // stop after the first level's passes
 };
-// One block (levels of at most kSmallOneMaxN vertices), or one cluster of 16
-// (8 where the device cannot co-schedule 16).  cudaErrorNotSupported: the
-// device cannot run it.
-cudaError_t launch_small_run(const SmallRunArgs& A, int mode, bool one, cudaStream_t st);
+// Blocks of the largest cluster the current device can run the small-run kernel
+// with (16, 8, or 0: none).  Opts the kernel in to its shared memory and
+// cluster size, which belong to the device's context: every engine asks for
+// itself before its first launch.
+int small_run_cluster(int mode);
+// On one cluster of ctas blocks, or with ctas = 1 on one block (levels of at
+// most kSmallOneMaxN vertices).
+cudaError_t launch_small_run(const SmallRunArgs& A, int mode, unsigned ctas, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
 // sort.cu

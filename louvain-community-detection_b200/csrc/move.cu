@@ -2877,47 +2877,49 @@ static cudaLaunchConfig_t small_run_config(cudaLaunchAttribute* at, unsigned cta
   return lc;
 }
 
-// Largest cluster the device can run the small-run kernel with (16, 8, or 0:
-// none), once per process.
 template <int MODE>
-static int small_run_cluster() {
-  static const int size = [] {
-    const void* f = (const void*)small_run_kernel<MODE>;
-    int found = 0;
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kSmallSmem) == cudaSuccess &&
-        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-            cudaSuccess) {
-      for (int c = kSmallCtas; c >= 8 && !found; c /= 2) {
-        cudaLaunchAttribute at[1];
-        const cudaLaunchConfig_t lc = small_run_config<MODE>(at, (unsigned)c, nullptr);
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, f, &lc) == cudaSuccess && n > 0) found = c;
-      }
+static int small_run_cluster_impl() {
+  const void* f = (const void*)small_run_kernel<MODE>;
+  int found = 0;
+  if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem) ==
+          cudaSuccess &&
+      cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+    for (int c = kSmallCtas; c >= 8 && !found; c /= 2) {
+      cudaLaunchAttribute at[1];
+      const cudaLaunchConfig_t lc = small_run_config<MODE>(at, (unsigned)c, nullptr);
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, f, &lc) == cudaSuccess && n > 0) found = c;
     }
-    cudaGetLastError();
-    return found;
-  }();
-  return size;
+  }
+  cudaGetLastError();
+  return found;
+}
+
+int small_run_cluster(int mode) {
+  switch (mode) {
+    case 0: return small_run_cluster_impl<0>();
+    case 1: return small_run_cluster_impl<1>();
+    case 2: return small_run_cluster_impl<2>();
+    case 3: return small_run_cluster_impl<3>();
+    default: return 0;
+  }
 }
 
 template <int MODE>
-static cudaError_t launch_small_run_impl(const SmallRunArgs& A, bool one, cudaStream_t st) {
-  const int most = small_run_cluster<MODE>();
-  if (!most) return cudaErrorNotSupported;
+static cudaError_t launch_small_run_impl(const SmallRunArgs& A, unsigned ctas, cudaStream_t st) {
   cudaLaunchAttribute at[1];
-  const cudaLaunchConfig_t lc = small_run_config<MODE>(at, one ? 1u : (unsigned)most, st);
+  const cudaLaunchConfig_t lc = small_run_config<MODE>(at, ctas, st);
   count_launches(1);
   return cudaLaunchKernelEx(&lc, small_run_kernel<MODE>, A,
-                            one ? kSmallOneMaxN : kSmallMaxN);
+                            ctas == 1 ? kSmallOneMaxN : kSmallMaxN);
 }
 
-cudaError_t launch_small_run(const SmallRunArgs& A, int mode, bool one, cudaStream_t st) {
+cudaError_t launch_small_run(const SmallRunArgs& A, int mode, unsigned ctas, cudaStream_t st) {
   switch (mode) {
-    case 0: return launch_small_run_impl<0>(A, one, st);
-    case 1: return launch_small_run_impl<1>(A, one, st);
-    case 2: return launch_small_run_impl<2>(A, one, st);
-    case 3: return launch_small_run_impl<3>(A, one, st);
+    case 0: return launch_small_run_impl<0>(A, ctas, st);
+    case 1: return launch_small_run_impl<1>(A, ctas, st);
+    case 2: return launch_small_run_impl<2>(A, ctas, st);
+    case 3: return launch_small_run_impl<3>(A, ctas, st);
     default: return cudaErrorInvalidValue;
   }
 }
