@@ -196,8 +196,15 @@ lv_status lv_engine_load_device(lv_engine *e, uint32_t n_vertices,
  * lv_graph_load_mtx (parallel host parse), then the device build.
  * lv_csr_from_edges_device: device in, device out on `stream`; d_cols and
  * d_weights_out need room for 2 * n_edges entries, d_offsets for
- * n_vertices + 1; *n_entries receives the entry count; scratch is
- * allocated and freed on the stream.                                      */
+ * n_vertices + 1; *n_entries receives the entry count.  Its scratch (about
+ * 32 bytes per edge line) is allocated and freed on the stream, from a pool
+ * that keeps up to 512 MiB of it per device for the next call (and for the
+ * loads above and lv_get_communities).  That memory is given back when an
+ * engine of the device is destroyed, when one of the library's allocations
+ * fails for want of memory (which is then tried again), and by
+ * lv_release_scratch, which a program that makes no engine calls when it
+ * needs the memory elsewhere, or before it ends the device's context
+ * (cudaDeviceReset).  Calls that are under way keep what they use.         */
 lv_status lv_engine_load_edges(lv_engine *e, uint32_t n_vertices, uint64_t n_edges,
                                const uint32_t *src, const uint32_t *dst,
                                const float *weights);
@@ -207,6 +214,7 @@ lv_status lv_csr_from_edges_device(uint32_t n_vertices, uint64_t n_edges,
                                    const float *d_weights, uint64_t *d_offsets,
                                    uint32_t *d_cols, float *d_weights_out,
                                    uint64_t *n_entries, void *stream);
+lv_status lv_release_scratch(int device);
 
 /* One phase of local moving on the current level (modularityOptimization,
  * modularity.cu:438-520).  *more = 1 when the first pass gained at least

@@ -80,17 +80,39 @@ struct AllocScope {
 std::atomic<unsigned long long> g_alloc_count{0};
 std::atomic<unsigned long long> g_alloc_fail_at{0};
 
+// An allocation that fails is tried again without the scratch that the sorts
+// keep between calls.
+template <class F>
+cudaError_t alloc_or_release(F alloc) {
+  cudaError_t e = alloc();
+  int dev = 0;
+  if (e != cudaErrorMemoryAllocation || cudaGetDevice(&dev) != cudaSuccess) return e;
+  cudaGetLastError();
+  release_sort_scratch(dev);
+  return alloc();
+}
+
 template <typename T>
 cudaError_t dalloc(T** p, size_t count) {
   *p = nullptr;
   const unsigned long long fail_at = g_alloc_fail_at.load(std::memory_order_relaxed);
-  if (fail_at && g_alloc_count.fetch_add(1, std::memory_order_relaxed) + 1 == fail_at)
-    return cudaErrorMemoryAllocation;
-  if (count == 0) count = 1;
-  if (t_alloc_stream && t_alloc_pool)
-    return cudaMallocFromPoolAsync((void**)p, count * sizeof(T), t_alloc_pool, t_alloc_stream);
-  if (t_alloc_stream) return cudaMallocAsync((void**)p, count * sizeof(T), t_alloc_stream);
-  return cudaMalloc((void**)p, count * sizeof(T));
+  const bool fails =
+      fail_at && g_alloc_count.fetch_add(1, std::memory_order_relaxed) + 1 == fail_at;
+  const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+  return alloc_or_release([&]() -> cudaError_t {
+    if (fails) return cudaErrorMemoryAllocation;
+    if (t_alloc_stream && t_alloc_pool)
+      return cudaMallocFromPoolAsync((void**)p, bytes, t_alloc_pool, t_alloc_stream);
+    if (t_alloc_stream) return cudaMallocAsync((void**)p, bytes, t_alloc_stream);
+    return cudaMalloc((void**)p, bytes);
+  });
+}
+
+// Outside the engine's pool, whatever the scope (fixed-size or freed with
+// cudaFree).
+template <typename T>
+cudaError_t device_malloc(T** p, size_t bytes) {
+  return alloc_or_release([&] { return cudaMalloc((void**)p, bytes); });
 }
 
 template <typename T>
@@ -737,7 +759,7 @@ lv_status ensure_capacity(lv_engine* E, uint32_t n, uint64_t e, bool need_input)
   B.g_cap = 0;
   const size_t scan_cap = std::max<size_t>(N1, partition_tmp_words(N)) + 1024;
   E->scan.bytes = scan_scratch_bytes(scan_cap);
-  CU(cudaMalloc(&E->scan.buf, E->scan.bytes));
+  CU(device_malloc(&E->scan.buf, E->scan.bytes));
   E->cap_n = n;
   E->cap_e = e;
   return LV_OK;
@@ -1935,9 +1957,9 @@ lv_status lv_engine_create(const lv_config* cfg, lv_engine** out) {
     }
     E->own_stream = true;
   }
-  if ((ce = cudaMalloc(&E->sc, sizeof(LevelScalars))) != cudaSuccess ||
-      (ce = cudaMalloc(&E->d_desc, sizeof(PassDesc))) != cudaSuccess ||
-      (ce = cudaMalloc(&E->loop_state, sizeof(LevelLoopState))) != cudaSuccess ||
+  if ((ce = device_malloc(&E->sc, sizeof(LevelScalars))) != cudaSuccess ||
+      (ce = device_malloc(&E->d_desc, sizeof(PassDesc))) != cudaSuccess ||
+      (ce = device_malloc(&E->loop_state, sizeof(LevelLoopState))) != cudaSuccess ||
       (ce = cudaMallocHost(&E->loop_host, sizeof(LevelLoopState))) != cudaSuccess ||
       (ce = cudaMallocHost(&E->sc_host, sizeof(LevelScalars))) != cudaSuccess ||
       (ce = cudaMallocHost(&E->h_counts, 32 * sizeof(uint32_t))) != cudaSuccess ||
@@ -3188,6 +3210,12 @@ lv_status lv_debug_fail_device_alloc(uint64_t n) {
   g_alloc_fail_at.store(0, std::memory_order_relaxed);
   g_alloc_count.store(0, std::memory_order_relaxed);
   g_alloc_fail_at.store(n, std::memory_order_relaxed);
+  return LV_OK;
+}
+
+lv_status lv_release_scratch(int device) {
+  if (device < 0) return fail(LV_ERR_ARG, "no such device");
+  release_sort_scratch(device);
   return LV_OK;
 }
 

@@ -575,7 +575,7 @@ template <typename K>
 cudaError_t radix_sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt,
                              uint64_t n, int key_bits, uint32_t* counts, ScanScratch& S,
                              cudaStream_t st, bool* result_in_alt);
-// Gives back the sorts' unused scratch on a device (kept between calls).
+// Gives back the scratch that the sorts keep between calls on a device.
 void release_sort_scratch(int device);
 // CSR of an edge list with the reference reader's layout (utils.cu:168-229):
 // every row in file order, an off-diagonal edge stored in both rows, a

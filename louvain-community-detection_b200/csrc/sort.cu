@@ -319,19 +319,19 @@ int bits_for(uint64_t max_key) {
 // the freed scratch back to the driver and the next call maps it again (CSR
 // of 12 M edges: 6.8 ms a call, 2.0 ms of it kernels).  The pool keeps at
 // most kKeepBytes of freed memory, the rest goes back at the next
-// synchronisation; release_sort_scratch() and a failed allocation give all
-// of it back.  Allocations are stream-ordered, so streams and threads may
-// share it.
+// synchronisation.  release_sort_scratch() gives all of it back: called when
+// an engine of the device ends, when an allocation fails (a sort's here, an
+// engine's in its own wrapper) and by lv_release_scratch.  It drops the pool
+// itself, so none outlives the device's context once its users have let go;
+// blocks in use stay valid until they are freed.  Allocations are
+// stream-ordered, so streams and threads may share the pool.
 constexpr uint64_t kKeepBytes = 512ull << 20;
 constexpr int kMaxDevices = 64;
-std::mutex g_pool_mu;
+std::mutex g_pool_mu;  // held over an allocation: the pool may be dropped
 cudaMemPool_t g_pool[kMaxDevices] = {};
 
-cudaError_t sort_pool(cudaMemPool_t* out) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= kMaxDevices) return cudaDeviceGetDefaultMemPool(out, dev);
+cudaError_t pool_alloc(void** p, size_t bytes, int dev, cudaStream_t st) {
+  if (dev < 0 || dev >= kMaxDevices) return cudaMallocAsync(p, bytes, st);
   std::lock_guard<std::mutex> lock(g_pool_mu);
   if (!g_pool[dev]) {
     cudaMemPoolProps props = {};
@@ -339,14 +339,14 @@ cudaError_t sort_pool(cudaMemPool_t* out) {
     props.handleTypes = cudaMemHandleTypeNone;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    cudaMemPool_t p = nullptr;
-    if ((e = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return e;
+    cudaMemPool_t pool = nullptr;
+    const cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return e;
     uint64_t keep = kKeepBytes;
-    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    g_pool[dev] = p;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    g_pool[dev] = pool;
   }
-  *out = g_pool[dev];
-  return cudaSuccess;
+  return cudaMallocFromPoolAsync(p, bytes, g_pool[dev], st);
 }
 
 // A sort's scratch: stream-ordered blocks, freed when it goes out of scope.
@@ -355,20 +355,22 @@ struct Scratch {
   void* blocks[8];
   int n = 0;
   explicit Scratch(cudaStream_t s) : st(s) {}
-  ~Scratch() {
+  ~Scratch() { release(); }
+  void release() {
     for (int i = 0; i < n; i++) cudaFreeAsync(blocks[i], st);
+    n = 0;
   }
   template <typename T>
   cudaError_t get(T** p, size_t count) {
-    cudaMemPool_t pool = nullptr;
-    cudaError_t e = sort_pool(&pool);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-    e = cudaMallocFromPoolAsync((void**)p, bytes, pool, st);
+    e = pool_alloc((void**)p, bytes, dev, st);
     if (e == cudaErrorMemoryAllocation) {  // the pool's unused blocks may be in the way
       cudaGetLastError();
-      cudaMemPoolTrimTo(pool, 0);
-      e = cudaMallocFromPoolAsync((void**)p, bytes, pool, st);
+      release_sort_scratch(dev);
+      e = pool_alloc((void**)p, bytes, dev, st);
     }
     if (e == cudaSuccess) blocks[n++] = *p;
     return e;
@@ -438,7 +440,8 @@ template cudaError_t radix_sort_pairs<uint64_t>(uint64_t*, uint32_t*, uint64_t*,
 void release_sort_scratch(int device) {
   if (device < 0 || device >= kMaxDevices) return;
   std::lock_guard<std::mutex> lock(g_pool_mu);
-  if (g_pool[device]) cudaMemPoolTrimTo(g_pool[device], 0);
+  if (g_pool[device]) cudaMemPoolDestroy(g_pool[device]);
+  g_pool[device] = nullptr;
 }
 
 cudaError_t csr_from_edges_device(uint32_t n, uint64_t m, const uint32_t* src,
@@ -497,6 +500,7 @@ cudaError_t csr_from_edges_device(uint32_t n, uint64_t m, const uint32_t* src,
   if ((e = cudaMemcpyAsync(bad_host, bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, st)) !=
       cudaSuccess)
     return e;
+  tmp.release();  // before the wait: afterwards the pool can give it back
   return counted_sync(st);
 }
 

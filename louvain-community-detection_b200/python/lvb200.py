@@ -167,6 +167,7 @@ _SIGS = {
     "lv_engine_load_mtx": (ctypes.c_int, [_VP, ctypes.c_char_p]),
     "lv_csr_from_edges_device": (ctypes.c_int, [_U32, _U64, _VP, _VP, _VP, _VP, _VP, _VP,
                                                 ctypes.POINTER(_U64), _VP]),
+    "lv_release_scratch": (ctypes.c_int, [ctypes.c_int]),
     "lv_get_communities": (ctypes.c_int, [_VP, _VP, ctypes.c_size_t,
                                           ctypes.POINTER(_U32)]),
     "lv_modularity_noalloc": (ctypes.c_int, [_U32, _VP, _VP, _VP, _VP, _VP,
@@ -268,6 +269,12 @@ def fail_device_alloc(n: int):
     """Fault injection for tests: the nth device allocation from now on
     fails as out-of-memory (0 switches it off)."""
     _check(lib().lv_debug_fail_device_alloc(n))
+
+
+def release_scratch(device: int = 0):
+    """Gives back the device memory that CSR builds and community listings
+    keep for the next one (at most 512 MiB)."""
+    _check(lib().lv_release_scratch(device))
 
 
 def launch_count() -> int:
