@@ -1259,6 +1259,9 @@ lv_status check_device_error(lv_engine* E) {
   if (E->sc_host->error == kErrBarrierTimeout) {
     return fail(LV_ERR_TIMEOUT, "a grid barrier wait of the level kernel gave up");
   }
+  if (E->sc_host->error == kErrUnionChunks) {
+    return fail(LV_ERR_STATE, "the union's entry chunks are out of step with its rows");
+  }
   if (E->sc_host->error) {
     return fail(LV_ERR_LIMIT, "a device hash table overflowed (bounded probe gave up)");
   }

@@ -341,9 +341,11 @@ struct LevelLoopState {
   unsigned long long phase_cnt[kPhaseKinds];
 };
 // LevelScalars::error values: a bounded hash probe gave up / a barrier wait
-// of the persistent level kernel gave up.
+// of the persistent level kernel gave up / the union sweep's chunk starts do
+// not fit its rows.
 constexpr uint32_t kErrTableFull = 1u;
 constexpr uint32_t kErrBarrierTimeout = 2u;
+constexpr uint32_t kErrUnionChunks = 3u;
 
 struct PassDesc {
   LevelView L;

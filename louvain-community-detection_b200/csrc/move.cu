@@ -1846,7 +1846,7 @@ __device__ __forceinline__ void union_sweep(const LevelView& L, const uint32_t* 
   const uint32_t lane = threadIdx.x & 31;
   while (c < c_end) {  // block-uniform: one graph's chunks of the range
     uint32_t g = 0, hi = L.n_graphs;  // the last graph starting at or before c
-    for (int round = 0; round < 7 && hi - g > 1; round++) {  // 32^7 > 2^32
+    while (hi - g > 1) {  // lane 0's candidate is g: a round leaves [g, g + step)
       const uint32_t step = (hi - g + 31) / 32, i = g + lane * step;
       const unsigned b = __ballot_sync(kFull, lane == 0 || (i < hi && U.start[i] <= c));
       g += (uint32_t)(__popc(b) - 1) * step;
@@ -1857,8 +1857,12 @@ __device__ __forceinline__ void union_sweep(const LevelView& L, const uint32_t* 
     const uint64_t e0 = L.off[v0], e1 = L.off[v1];
     const uint32_t chunks = (uint32_t)((e1 - e0 + kUnionChunk - 1) / kUnionChunk);
     const uint32_t c1 = min(c_end, first + chunks);
-    if (c < first || c1 <= c) {  // the starts are out of step with the rows
-      if (threadIdx.x == 0) atomicExch(&L.sc->error, kErrTableFull);
+    // The starts were scanned from these same offsets before the first sweep
+    // after every change of the active set, which nothing changes in between,
+    // so graph g holds chunk c and the loop moves on.  Checked all the same: a
+    // state that did not fit would otherwise loop here without end.
+    if (c < first || c1 <= c) {
+      if (threadIdx.x == 0) atomicExch(&L.sc->error, kErrUnionChunks);
       return;
     }
     const uint64_t j1 = min(e1, e0 + (uint64_t)(c1 - first) * kUnionChunk);
