@@ -199,7 +199,8 @@ lv_status lv_engine_load_device(lv_engine *e, uint32_t n_vertices,
  * n_vertices + 1; *n_entries receives the entry count.  Its scratch (about
  * 32 bytes per edge line) is allocated and freed on the stream, from a pool
  * that keeps up to 512 MiB of it per device for the next call (and for the
- * loads above and lv_get_communities).  That memory is given back when an
+ * loads above and lv_get_communities); what is above that goes back when the
+ * stream is next waited for.  The memory kept is given back when an
  * engine of the device is destroyed, when one of the library's allocations
  * fails for want of memory (which is then tried again), and by
  * lv_release_scratch, which a program that makes no engine calls when it

@@ -318,12 +318,13 @@ int bits_for(uint64_t max_key) {
 // the first use: with the device's default pool every synchronisation gives
 // the freed scratch back to the driver and the next call maps it again (CSR
 // of 12 M edges: 6.8 ms a call, 2.0 ms of it kernels).  The pool keeps at
-// most kKeepBytes of freed memory, the rest goes back at the next
+// most kKeepBytes of freed memory, the rest goes back at the stream's next
 // synchronisation.  release_sort_scratch() gives all of it back: called when
 // an engine of the device ends, when an allocation fails (a sort's here, an
-// engine's in its own wrapper) and by lv_release_scratch.  It drops the pool
-// itself, so none outlives the device's context once its users have let go;
-// blocks in use stay valid until they are freed.  Allocations are
+// engine's in its own wrapper) and by lv_release_scratch.  It drops the pool:
+// trimming one gives nothing back while the frees queued after a call's wait
+// have not been waited for, and a pool must not outlive the device's context.
+// Blocks in use stay valid until they are freed.  Allocations are
 // stream-ordered, so streams and threads may share the pool.
 constexpr uint64_t kKeepBytes = 512ull << 20;
 constexpr int kMaxDevices = 64;
@@ -355,10 +356,8 @@ struct Scratch {
   void* blocks[8];
   int n = 0;
   explicit Scratch(cudaStream_t s) : st(s) {}
-  ~Scratch() { release(); }
-  void release() {
+  ~Scratch() {
     for (int i = 0; i < n; i++) cudaFreeAsync(blocks[i], st);
-    n = 0;
   }
   template <typename T>
   cudaError_t get(T** p, size_t count) {
@@ -500,7 +499,6 @@ cudaError_t csr_from_edges_device(uint32_t n, uint64_t m, const uint32_t* src,
   if ((e = cudaMemcpyAsync(bad_host, bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, st)) !=
       cudaSuccess)
     return e;
-  tmp.release();  // before the wait: afterwards the pool can give it back
   return counted_sync(st);
 }
 
