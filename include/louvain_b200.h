@@ -412,7 +412,8 @@ void lv_serve_destroy(lv_server *s);
  * choice changes speed only.  Variants: G-lane groups with one entry per
  * lane (LV_KERNEL_LANES4/8/16/32: degree <= G), a warp per vertex with a
  * 128-slot shared table (LV_KERNEL_WARP128: <= 84), four warps per vertex
- * with a 512-slot one (LV_KERNEL_WARP512: <= 319) and a block per vertex with a 4096-slot table (LV_KERNEL_BLOCK: <= 2048).
+ * with a 512-slot one (LV_KERNEL_WARP512: <= 319) and a block per vertex
+ * with a 4096-slot one (LV_KERNEL_BLOCK: <= 2048).
  * lv_autotune times every fitting variant of every non-empty bucket on the
  * loaded graph's current level (proposals only; the state is unchanged)
  * and keeps the fastest; the engine uses its tuning until changed.        */

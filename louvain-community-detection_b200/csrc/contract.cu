@@ -264,7 +264,8 @@ __global__ void g_fill_kernel(const uint32_t* __restrict__ counts,
 // members' range (four loads), so a warp takes up to 32 communities at a
 // time, a lane each one's chain, and merges those that have entries (an
 // isolated vertex stays a community without any at every level: half of
-// R-MAT 24's, which took 4.6 ms a level by themselves; 0.25 ms now; R-MAT 20's levels 151 -> 17 us).
+// R-MAT 24's, which took 4.6 ms a level by themselves; 0.25 ms now; R-MAT 20's
+// levels 151 -> 17 us).
 // Dealt round robin: large communities often have consecutive ids.
 // S: type of a table's sums -- FP64, or 32-bit integers on a level of whole
 // weights (LevelScalars::whole; exact either way), which shared memory adds
@@ -1008,6 +1009,10 @@ cudaError_t contract_back(const LevelView& L, uint64_t nnz, ContractBuffers& B,
   C.tw = B.tw;
   C.new_deg = B.new_deg;
   C.err = &L.sc->error;
+  // Written by the level's init.  A level whose passes the small-run kernel ran
+  // has none: the flag is then an earlier level's of the same graph, whose
+  // weights stay whole, and their total the same, when they are added up, or 0
+  // from the load.
   C.whole = &L.sc->whole;
 
   if (cntW) {

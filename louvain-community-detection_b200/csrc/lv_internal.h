@@ -445,8 +445,9 @@ DispatchArgs dispatch_args(const uint32_t* order, const DispatchPlan& P, const u
 // order[].
 // Move kernel variants a bucket can run on: G-lane groups (one entry per
 // lane, degree <= G), a warp with a 128-slot shared table, a block of four
-// warps with a 512-slot one, a block of eight with a 4096-slot one.  All give the same proposals; they differ in how
-// the work maps onto the SMs, which the autotuner measures.
+// warps with a 512-slot one, a block of eight with a 4096-slot one.  All give
+// the same proposals; they differ in how the work maps onto the SMs, which the
+// autotuner measures.
 enum MoveVariant : uint8_t {
   KV_SMALL4 = 0,
   KV_SMALL8 = 1,

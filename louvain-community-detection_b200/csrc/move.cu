@@ -30,16 +30,18 @@
 //     the lowest community id wins ties deterministically.
 //   * deg <= 32: G lanes per vertex (G = 4, 8, 16, 32), one edge per lane;
 //     equal communities in a group are found with G - 1 shuffles (4, 8) or
-//     through slots in shared memory (16, 32).  (__match_any_sync costs about one step per distinct
-//     value in the warp, and at level 0 all 32 values are distinct.)
+//     through slots in shared memory (16, 32).  (__match_any_sync costs about
+//     one step per distinct value in the warp, and at level 0 all 32 values
+//     are distinct.)
 //     32 < deg <= 84: one warp per vertex, open-addressing table in shared
 //     memory.  deg <= 319: a block of four warps per vertex, 512 slots.
 //     319 < deg <= 2048: a block of eight, 4096 slots.  deg > 2048: one
 //     block per (vertex, hash partition of its neighbour communities),
 //     4096-slot shared table, the partitions' best candidates merged with
-//     one 64-bit atomicMax each -- no global hash table, whatever the degree.  Shared tables are self-cleaning: a row
-//     uses the first slots of its table (a power of two >= 1.5 x its
-//     degree), and the candidate scan clears the slots it reads.
+//     one 64-bit atomicMax each -- no global hash table, whatever the degree.
+//     Shared tables are self-cleaning: a row uses the first slots of its table
+//     (a power of two >= 1.5 x its degree), and the candidate scan clears the
+//     slots it reads.
 //   * Community totals are updated incrementally by the moved vertices
 //     only (FP64 atomics), instead of a full recount after every bucket.
 #include "lv_internal.h"
@@ -341,8 +343,7 @@ __device__ __forceinline__ uint32_t table_claim(uint32_t* keys, uint32_t mask, u
 // integers by itself; an FP64 add is a loop of load, add and compare-and-swap,
 // on which lanes that meet in one community serialise (R-MAT 20, FP64 gains:
 // block kernel 525 -> 295 us a launch, hub merge 345 -> 193, warp kernel
-// 113 -> 108; R-MAT 24:
-// 3,310 -> 2,380, 7,860 -> 6,220, 1,200 -> 1,150).
+// 113 -> 108; R-MAT 24: 3,310 -> 2,380, 7,860 -> 6,220, 1,200 -> 1,150).
 template <class S>
 __device__ __forceinline__ S to_sum(float w) {
   return (S)w;
@@ -734,8 +735,9 @@ __device__ __forceinline__ typename BestOf<PREC>::T eval_claims(const LevelView&
   return best;
 }
 
-// 32 < deg <= 319: one warp per vertex, T-slot table per warp.  All of a
-// row's loads (at most MAXW waves of 32) are issued before any insertion,
+// 32 < deg <= 84 (the small-run and persistent level kernels: <= 319): one
+// warp per vertex, T-slot table per warp.  All of a row's loads (at most MAXW
+// waves of 32) are issued before any insertion,
 // so a vertex costs one memory latency chain instead of one per wave.  nw:
 // the block's warps that have a table (its first ones).
 template <int T, int MAXW, int MODE, class S, bool COHERENT>
@@ -1675,9 +1677,9 @@ __global__ void __launch_bounds__(kThreads)
   RowSumOp op;
   dispatch_units(L, A, op, red);
   if (L.gid) op.finish(L);
-  // singleton state (modularity.cu:459-462), and for a single graph the
-  // pass-start communities of the incremental sweep and the row of every
-  // entry (the pass loop's flat modularity sweep).  A warp takes 32
+  // singleton state (modularity.cu:459-462), the row of every entry (the pass
+  // loop's flat modularity sweeps), and for a single graph the pass-start
+  // communities of the incremental sweep.  A warp takes 32
   // consecutive ids, a lane each id's state and bounds, then writes the 32
   // rows' entry rows one row after another, 32 entries per store.
   const uint32_t lane = threadIdx.x & 31;
